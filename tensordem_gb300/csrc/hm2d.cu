@@ -28,7 +28,7 @@
 #include <string>
 #include <vector>
 
-#include "hm2d_dev.cuh"
+#include "hm2d_run.cuh"
 
 // ===========================================================================
 // Host engine
@@ -318,6 +318,10 @@ struct Engine final : EngineBase {
   int vgrid[kVariants] = {};
   int nwarp_slots = 0;
   int sgrid = 1;  // grid of the pipelined strain kernel (FP32 engines with bonds)
+  // resident step kernel (variant 0's step loop): discs per block, grid, build
+  RunFn<T> run = nullptr;
+  int run_pb = 0, run_grid = 0, run_threads = 0;
+  size_t run_smem = 0;
   bool primed = false;
   bool has_state = false;
   bool graph_on = true;
@@ -423,7 +427,8 @@ struct Engine final : EngineBase {
                               kStrainSmem));
       sgrid = std::max(1, std::min((int)((n + kStrainBlock - 1) / kStrainBlock), per_sm * sms));
     }
-    int rc = TDEM_OK;
+    int rc = plan_run(dev, sms);
+    if (rc) return rc;
     for (int b = 0; b < 2 && !rc; ++b) {
       if ((rc = alloc(&B.pos[b], n)) || (rc = alloc(&B.vel[b], n)) || (rc = alloc(&B.head[b], n)) ||
           (rc = alloc(&B.orig[b], n)) || (rc = alloc(&B.whist[b], 4 * n)) ||
@@ -438,7 +443,7 @@ struct Engine final : EngineBase {
         (rc = alloc(&B.tmp_off, n)) || (rc = alloc(&B.diss_part, (size_t)nwarp_slots)) ||
         (rc = alloc(&B.peek_part, (size_t)nblocks * 12)) || (rc = alloc(&B.peek_vel, n)) ||
         (rc = alloc(&B.peek_force, n)) || (rc = alloc(&B.ctl, 1)) || (rc = alloc(&B.invperm, n)) ||
-        (rc = alloc(&B.frac_part, (size_t)nwarp_slots)) || (rc = alloc(&B.ind_part, 6 * (size_t)nwarp_slots)) ||
+        (rc = alloc(&B.frac_part, (size_t)nwarp_slots)) || (rc = alloc(&B.ind_part, 8 * (size_t)nwarp_slots)) ||
         (rc = alloc(&B.load, 2 * (size_t)std::max(P.load_cap, 1))))
       return rc;
     if (P.BMAX > 0) {
@@ -460,6 +465,48 @@ struct Engine final : EngineBase {
     TDEM_CUDA_TRY(&err, cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
     return TDEM_OK;
   }
+
+  // The shape of the resident step kernel, if the engine fits one disc per
+  // thread of the chip. One block while that costs no more than a grid
+  // barrier; else blocks of at least 128 discs (one warp per scheduler), as
+  // many as the discs need, one per SM; the big build only when the other
+  // does not hold them.
+  int plan_run(int dev, int sms) {
+    int smem_max = 0, coop = 0;
+    TDEM_CUDA_TRY(&err, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    TDEM_CUDA_TRY(&err, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    const bool f = feat();
+    if (sum64 || !coop) return TDEM_OK;
+    smem_max -= 1024;                                  // the kernel's static shared memory
+    const int extra = f && P.irad > T(0) ? 32 : 0;     // the indenter's helper warp
+    auto warps = [](long long n) { return (int)((n + 31) / 32) * 32; };
+    for (int build = 0; build < 3; ++build) {
+      const bool local = build == 0, big = build == 2;
+      int most = run_block<T>(f, big) - extra;
+      if (local) most = std::min(most, f ? kRunLocalBonds : kRunLocal);
+      const int pb = local ? warps(P.n) : std::max(std::min(kRunDiscs, most), warps((P.n + sms - 1) / sms));
+      if (pb > most) continue;
+      const size_t smem = run_layout<T>(P.W, f ? P.BMAX : 0, pb, local ? 1 : 0, P.n).total;
+      if (smem > (size_t)smem_max) continue;
+      RunFn<T> fn = run_fn<T>(f, local, big);
+      int per_sm = 0;
+      TDEM_CUDA_TRY(&err, cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+      TDEM_CUDA_TRY(&err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn),
+                                                                        pb + extra, smem));
+      if (per_sm < 1) continue;
+      run = fn;
+      run_pb = pb;
+      run_grid = (P.n + pb - 1) / pb;
+      run_threads = pb + extra;
+      run_smem = smem;
+      break;
+    }
+    return TDEM_OK;
+  }
+
+  // The step graph loops around the resident kernel.
+  bool resident() const { return run && variant == 0; }
 
   bool feat() const { return P.BMAX > 0 || P.irad > T(0); }
   // launch shape of a variant's step kernel (the FP64-sum form has one shape)
@@ -515,39 +562,53 @@ struct Engine final : EngineBase {
     return TDEM_OK;
   }
 
-  // Adds `kernel -> IF(h) { rebuild pipeline }` to graph g.
+  // Adds `step kernel (resident: steps) -> IF(h) { rebuild pipeline }` to graph g.
   int add_step_and_rebuild(cudaGraph_t g, const cudaGraphNode_t* dep, size_t ndep,
                            cudaGraphConditionalHandle h, cudaGraphConditionalHandle hl, int cond_bits) {
-    int prim = 1;
-    StepHint nohint{};
-    void* args[] = {&P, &B, &h, &hl, &cond_bits, &prim, &nohint};
-    cudaKernelNodeParams kp = {};
-    kp.func = reinterpret_cast<void*>(step_fn<T>(variant, kStep, feat(), sum64));
-    kp.gridDim = dim3((unsigned)vgrid[variant]);
-    kp.blockDim = dim3((unsigned)block_of(variant));
-    kp.sharedMemBytes = (unsigned)smem_of(variant);
-    kp.kernelParams = args;
-    cudaGraphNode_t snode;
-    if (P.BMAX > 0) {
-      void* sargs[] = {&P, &B};
-      cudaKernelNodeParams sk = {};
-      if constexpr (sizeof(T) == 4) {
-        sk.func = reinterpret_cast<void*>(&strain_kernel_async<T>);
-        sk.gridDim = dim3((unsigned)sgrid);
-        sk.blockDim = dim3(kStrainBlock);
-        sk.sharedMemBytes = (unsigned)kStrainSmem;
-      } else {
-        sk.func = reinterpret_cast<void*>(&strain_kernel<T>);
-        sk.gridDim = grid_n();
-        sk.blockDim = dim3(kThreads);
-      }
-      sk.kernelParams = sargs;
-      TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&snode, g, dep, ndep, &sk));
-      dep = &snode;
-      ndep = 1;
-    }
     cudaGraphNode_t knode;
-    TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&knode, g, dep, ndep, &kp));
+    if (resident()) {
+      void* args[] = {&P, &B, &h, &hl, &cond_bits, &run_pb};
+      cudaKernelNodeParams kp = {};
+      kp.func = reinterpret_cast<void*>(run);
+      kp.gridDim = dim3((unsigned)run_grid);
+      kp.blockDim = dim3((unsigned)run_threads);
+      kp.sharedMemBytes = (unsigned)run_smem;
+      kp.kernelParams = args;
+      TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&knode, g, dep, ndep, &kp));
+      cudaKernelNodeAttrValue coop = {};
+      coop.cooperative = 1;
+      TDEM_CUDA_TRY(&err, cudaGraphKernelNodeSetAttribute(knode, cudaLaunchAttributeCooperative, &coop));
+    } else {
+      int prim = 1;
+      StepHint nohint{};
+      void* args[] = {&P, &B, &h, &hl, &cond_bits, &prim, &nohint};
+      cudaKernelNodeParams kp = {};
+      kp.func = reinterpret_cast<void*>(step_fn<T>(variant, kStep, feat(), sum64));
+      kp.gridDim = dim3((unsigned)vgrid[variant]);
+      kp.blockDim = dim3((unsigned)block_of(variant));
+      kp.sharedMemBytes = (unsigned)smem_of(variant);
+      kp.kernelParams = args;
+      cudaGraphNode_t snode;
+      if (P.BMAX > 0) {
+        void* sargs[] = {&P, &B};
+        cudaKernelNodeParams sk = {};
+        if constexpr (sizeof(T) == 4) {
+          sk.func = reinterpret_cast<void*>(&strain_kernel_async<T>);
+          sk.gridDim = dim3((unsigned)sgrid);
+          sk.blockDim = dim3(kStrainBlock);
+          sk.sharedMemBytes = (unsigned)kStrainSmem;
+        } else {
+          sk.func = reinterpret_cast<void*>(&strain_kernel<T>);
+          sk.gridDim = grid_n();
+          sk.blockDim = dim3(kThreads);
+        }
+        sk.kernelParams = sargs;
+        TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&snode, g, dep, ndep, &sk));
+        dep = &snode;
+        ndep = 1;
+      }
+      TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&knode, g, dep, ndep, &kp));
+    }
     cudaGraphNodeParams ip = {};
     ip.type = cudaGraphNodeTypeConditional;
     ip.conditional.handle = h;
@@ -564,14 +625,16 @@ struct Engine final : EngineBase {
     return TDEM_OK;
   }
 
-  // Two graphs: one step (kernel -> IF rebuild), and n steps
-  // (set target -> WHILE { kernel -> IF rebuild }).
+  // Two graphs: one step (kernel -> IF rebuild), unless the kernel is resident,
+  // and n steps (set target -> WHILE { kernel -> IF rebuild }).
   int build_graph() {
     int rc;
-    TDEM_CUDA_TRY(&err, cudaGraphCreate(&graph1, 0));
-    TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_reb1, graph1, 0, cudaGraphCondAssignDefault));
-    if ((rc = add_step_and_rebuild(graph1, nullptr, 0, h_reb1, 0, 1))) return rc;
-    TDEM_CUDA_TRY(&err, cudaGraphInstantiate(&exec1, graph1, 0));
+    if (!resident()) {
+      TDEM_CUDA_TRY(&err, cudaGraphCreate(&graph1, 0));
+      TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_reb1, graph1, 0, cudaGraphCondAssignDefault));
+      if ((rc = add_step_and_rebuild(graph1, nullptr, 0, h_reb1, 0, 1))) return rc;
+      TDEM_CUDA_TRY(&err, cudaGraphInstantiate(&exec1, graph1, 0));
+    }
 
     TDEM_CUDA_TRY(&err, cudaGraphCreate(&graph, 0));
     TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_loop, graph, 1, cudaGraphCondAssignDefault));
@@ -596,6 +659,24 @@ struct Engine final : EngineBase {
     TDEM_CUDA_TRY(&err, cudaGraphInstantiate(&exec, graph, 0));
     exec_target = 1;
     return TDEM_OK;
+  }
+
+  // The step graph, built when it is missing. Where a cooperative node cannot
+  // be instantiated the loop takes the one-step kernel; where no conditional
+  // graph can, steps are plain launches (same results).
+  void ensure_graph() {
+    if (!graph_on || graph_failed || exec) return;
+    if (build_graph() == TDEM_OK) return;
+    destroy_graphs();
+    if (resident()) {
+      run = nullptr;
+      cudaGetLastError();
+      if (build_graph() == TDEM_OK) return;
+      destroy_graphs();
+    }
+    graph_error = err;
+    graph_failed = true;
+    cudaGetLastError();
   }
 
   // Point the n-step graph's target node at n (only when n changes).
@@ -636,38 +717,27 @@ struct Engine final : EngineBase {
     if (n <= 0) {
       // no step: build the step graph for the current variant now, so that
       // the next call does not (instantiating it takes ~0.5 s)
-      if (graph_on && !graph_failed && !exec && build_graph() != TDEM_OK) {
-        graph_error = err;
-        graph_failed = true;
-        destroy_graphs();
-        cudaGetLastError();
-      }
+      ensure_graph();
       return TDEM_OK;
     }
     mirror_ok = false;  // rebuild decisions inside the step graph are the device's
-    if (!primed) {
+    ensure_graph();
+    const bool in_graph = graph_on && exec;
+    if (!primed && !(in_graph && resident())) {  // the resident kernel primes by itself
       int rc = prime(s);
       if (rc) return rc;
       --n;
       if (n == 0) return TDEM_OK;
     }
-    if (graph_on && !graph_failed && !exec) {
-      if (build_graph() != TDEM_OK) {
-        // fall back to plain launches (same kernels, same results)
-        graph_error = err;
-        graph_failed = true;
-        destroy_graphs();
-        cudaGetLastError();
-      }
-    }
-    if (graph_on && exec) {
-      if (n == 1) {
+    if (in_graph) {
+      if (n == 1 && exec1) {
         TDEM_CUDA_TRY(&err, cudaGraphLaunch(exec1, s));
         return TDEM_OK;
       }
       int rc = set_graph_target(n);
       if (rc) return rc;
       TDEM_CUDA_TRY(&err, cudaGraphLaunch(exec, s));
+      primed = true;
       return TDEM_OK;
     }
     for (long long k = 0; k < n; ++k) {

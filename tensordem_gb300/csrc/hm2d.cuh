@@ -111,6 +111,13 @@ constexpr unsigned kBondBroken = 1u << 31;
 constexpr int kBondModeShift = 29;
 constexpr int kMaxBondSlots = 8;
 
+// One grid barrier of the resident step kernel: arrivals, and what the blocks
+// agree on with it (largest |v|^2 as float bits, a non-finite state). A waiter
+// reads all of it in one 16-byte load.
+struct alignas(16) GridWord {
+  unsigned count, vmax2_bits, bad, pad;
+};
+
 // Device control block: buffer parities, the rebuild trigger and status.
 struct Ctl {
   int sp;                  // current pos/vel/hist buffer
@@ -139,6 +146,11 @@ struct Ctl {
   int since;               // steps since the last rebuild
   int key_hi;              // dead-particle key: one past the highest allocated cell key
   int tile_next;           // next tile chunk handed out by the (first) step launch
+  // resident step kernel: barrier k of the engine uses word k % 3 (`epoch`
+  // counts them across launches), zeroed one barrier ahead
+  unsigned epoch;
+  unsigned entries[2];     // indenter partials of the even and odd evaluations
+  alignas(128) GridWord word[3];
 };
 
 // Batched engine: per-instance state word (low byte: Status bits of the

@@ -250,32 +250,32 @@ struct WindowFetch {
   __device__ __forceinline__ V4<T> v(int j) const { return in(j) ? svel[(j - off) & mask] : vel[j]; }
 };
 
-// One candidate slot of particle i (partner j at position q): contact test,
-// history update in place, force and torque accumulation.
-template <class T, int MODE, class F, class A>
-__device__ __forceinline__ void do_slot(const Params<T>& P, const F& fetch,
-                                        V2<T>* __restrict__ hist, int i, int j, int s, size_t slot,
-                                        const V4<T>& p, const V4<T>& v, const V4<T>& q, unsigned mask,
-                                        unsigned& nmask, A& fx, A& fy, A& tq, T& diss, T& un,
-                                        T& ut, int primed) {
+// The geometry of particle i's candidate j at position q, from canonically
+// ordered operands; the pair touches when d2 < rs^2.
+template <class T>
+__device__ __forceinline__ Geo<T> slot_geo(const Params<T>& P, int i, int j, const V4<T>& p, const V4<T>& q) {
+  const bool owner = i < j;
+  return pair_geo<T>(P, owner ? p : q, owner ? q : p);
+}
+
+// A touching candidate slot s of particle i, its operands loaded: partner
+// position q and velocity w, stored history xi0. History update into `slot`,
+// force and torque accumulation.
+template <class T, int MODE, class A>
+__device__ __forceinline__ void touching_slot(const Params<T>& P, V2<T>* slot, int i, int j, int s, const Geo<T>& g,
+                                              const V4<T>& p, const V4<T>& v, const V4<T>& q, const V4<T>& w,
+                                              const V2<T>& xi0, bool stored, unsigned& nmask, A& fx, A& fy, A& tq,
+                                              T& diss, T& un, T& ut, int primed) {
   constexpr bool COMMIT = MODE != kPeek;
   const bool owner = i < j;
   const V4<T>& a = owner ? p : q;
   const V4<T>& b = owner ? q : p;
-  const Geo<T> g = pair_geo<T>(P, a, b);
-  const bool stored = (mask >> s) & 1u;
-  if (!(g.d2 < g.rs * g.rs)) {
-    if (COMMIT && stored) hist[slot] = V2<T>{T(0), T(0)};  // contact opened: reset
-    return;
-  }
-  const V4<T> w = fetch.v(j);
   const V4<T>& va = owner ? v : w;
   const V4<T>& vb = owner ? w : v;
-  const V2<T> xi0 = stored ? hist[slot] : V2<T>{T(0), T(0)};
   const PairOut<T> o = pair_force<T>(P, g, a, va, b, vb, xi0);
   if (COMMIT) {
     const bool nz = (o.xi.x != T(0)) || (o.xi.y != T(0));
-    if (nz || stored) hist[slot] = o.xi;
+    if (nz || stored) *slot = o.xi;
     nmask |= (nz ? 1u : 0u) << s;
   }
   if (owner) {
@@ -289,6 +289,26 @@ __device__ __forceinline__ void do_slot(const Params<T>& P, const F& fetch,
     fy.add(-o.fy);
   }
   tq.add(p.z * o.cr);
+}
+
+// One candidate slot of particle i (partner j at position q): contact test,
+// history update in place, force and torque accumulation.
+template <class T, int MODE, class F, class A>
+__device__ __forceinline__ void do_slot(const Params<T>& P, const F& fetch,
+                                        V2<T>* __restrict__ hist, int i, int j, int s, size_t slot,
+                                        const V4<T>& p, const V4<T>& v, const V4<T>& q, unsigned mask,
+                                        unsigned& nmask, A& fx, A& fy, A& tq, T& diss, T& un,
+                                        T& ut, int primed) {
+  constexpr bool COMMIT = MODE != kPeek;
+  const Geo<T> g = slot_geo<T>(P, i, j, p, q);
+  const bool stored = (mask >> s) & 1u;
+  if (!(g.d2 < g.rs * g.rs)) {
+    if (COMMIT && stored) hist[slot] = V2<T>{T(0), T(0)};  // contact opened: reset
+    return;
+  }
+  const V4<T> w = fetch.v(j);
+  const V2<T> xi0 = stored ? hist[slot] : V2<T>{T(0), T(0)};
+  touching_slot<T, MODE>(P, hist + slot, i, j, s, g, p, v, q, w, xi0, stored, nmask, fx, fy, tq, diss, un, ut, primed);
 }
 
 // Symmetric 2x2 pseudo-inverse (eigen-decomposition, cutoff 2 eps sigma_max).
@@ -764,6 +784,61 @@ __device__ __forceinline__ float add_prod_comp(float x, float& r, float a, float
   return s2;
 }
 
+// The walls of a disc in a border cell, each with its history slot.
+template <class T, int MODE, class A>
+__device__ __forceinline__ void wall_contacts(const Params<T>& P, V2<T>* wh, int i, const V4<T>& p, const V4<T>& v,
+                                              A& fx, A& fy, A& tq, ThreadLedger<T>& L, int primed) {
+  constexpr bool COMMIT = MODE != kPeek;
+  if (!P.walls || !(v.w > T(0))) return;
+  const int c = lane_to_cell(p.w);
+  const int cx = c & 0xFFFF, cy = c >> 16;
+  if (!(cx == 0 || cx == P.ncx - 1 || cy == 0 || cy == P.ncy - 1)) return;
+  const size_t n = (size_t)P.n;
+  const bool old_xi = (MODE == kPeek && !primed);
+  if ((P.walls & 1) && cx == 0)
+    wall_contact<T, COMMIT>(P, T(1), T(0), p.x, p, v, &wh[i], fx, fy, tq, L.diss, L.un, L.ut, old_xi);
+  if ((P.walls & 2) && cx == P.ncx - 1)
+    wall_contact<T, COMMIT>(P, T(-1), T(0), P.cell - p.x, p, v, &wh[n + i], fx, fy, tq, L.diss, L.un, L.ut, old_xi);
+  if ((P.walls & 4) && cy == 0)
+    wall_contact<T, COMMIT>(P, T(0), T(1), p.y, p, v, &wh[2 * n + i], fx, fy, tq, L.diss, L.un, L.ut, old_xi);
+  if ((P.walls & 8) && cy == P.ncy - 1)
+    wall_contact<T, COMMIT>(P, T(0), T(-1), P.cell - p.y, p, v, &wh[3 * n + i], fx, fy, tq, L.diss, L.un, L.ut,
+                            old_xi);
+}
+
+// The velocity-Verlet update of one disc from its accelerations.
+template <class T>
+struct Moved {
+  V4<T> pos, vel;
+  float2 rem;
+};
+
+template <class T, int MODE>
+__device__ __forceinline__ Moved<T> move_particle(const Params<T>& P, const V4<T>& p, const V4<T>& v, float2 rem, T ax,
+                                                  T ay, T al, int primed, ThreadLedger<T>& L) {
+  T vx, vy, om;
+  if (MODE == kPrime || (MODE == kBatch && !primed)) {
+    vx = v.x + P.half_dt * ax;
+    vy = v.y + P.half_dt * ay;
+    om = v.z + P.half_dt * al;
+  } else {
+    vx = (v.x + P.half_dt * ax) + P.half_dt * ax;
+    vy = (v.y + P.half_dt * ay) + P.half_dt * ay;
+    om = (v.z + P.half_dt * al) + P.half_dt * al;
+  }
+  T ox, oy;
+  if (sizeof(T) == 4 && P.prem) {
+    ox = (T)add_prod_comp((float)p.x, rem.x, (float)P.dt, (float)vx);
+    oy = (T)add_prod_comp((float)p.y, rem.y, (float)P.dt, (float)vy);
+  } else {
+    ox = p.x + P.dt * vx;
+    oy = p.y + P.dt * vy;
+  }
+  L.vmax2 = fmaxf(L.vmax2, (float)(vx * vx + vy * vy));
+  if (!(isfinite(ox) && isfinite(oy) && isfinite(vx) && isfinite(vy) && isfinite(om))) L.bad = true;
+  return Moved<T>{V4<T>{ox, oy, p.z, p.w}, V4<T>{vx, vy, om, v.w}, rem};
+}
+
 // Everything one particle does in one evaluation: its candidate slots, the
 // walls, and (committing modes) the velocity-Verlet update into the other
 // buffers. p, v, hd are the particle's own loads (already issued).
@@ -856,24 +931,7 @@ __device__ __forceinline__ void process_particle_q(const Params<T>& P, const Buf
   if (COMMIT && nmask != mask) B.head[lp][i].x = (hd.x & 0xFFu) | (nmask << 8);
   const int c = lane_to_cell(p.w);
   if (FEAT && P.irad > T(0)) indenter_contact<T>(P, eval, p, v, fx, fy, L);
-  if (P.walls && v.w > T(0)) {
-    const int cx = c & 0xFFFF, cy = c >> 16;
-    if ((cx == 0 || cx == P.ncx - 1 || cy == 0 || cy == P.ncy - 1)) {
-      V2<T>* wh = B.whist[lp];
-      const bool old_xi = (MODE == kPeek && !primed);
-      if ((P.walls & 1) && cx == 0)
-        wall_contact<T, COMMIT>(P, T(1), T(0), p.x, p, v, &wh[i], fx, fy, tq, L.diss, L.un, L.ut, old_xi);
-      if ((P.walls & 2) && cx == P.ncx - 1)
-        wall_contact<T, COMMIT>(P, T(-1), T(0), P.cell - p.x, p, v, &wh[(size_t)n + i], fx, fy, tq, L.diss, L.un,
-                                L.ut, old_xi);
-      if ((P.walls & 4) && cy == 0)
-        wall_contact<T, COMMIT>(P, T(0), T(1), p.y, p, v, &wh[(size_t)2 * n + i], fx, fy, tq, L.diss, L.un, L.ut,
-                                old_xi);
-      if ((P.walls & 8) && cy == P.ncy - 1)
-        wall_contact<T, COMMIT>(P, T(0), T(-1), P.cell - p.y, p, v, &wh[(size_t)3 * n + i], fx, fy, tq, L.diss,
-                                L.un, L.ut, old_xi);
-    }
-  }
+  wall_contacts<T, MODE>(P, B.whist[lp], i, p, v, fx, fy, tq, L, primed);
   const T Fx = fx.get(), Fy = fy.get(), Tz = tq.get();
   const T inv_m = v.w;  // 0 for a clamped disc
   const bool free = inv_m > T(0);
@@ -901,30 +959,10 @@ __device__ __forceinline__ void process_particle_q(const Params<T>& P, const Buf
     // the potential energy.
     if (sizeof(T) == 4 && P.prem) L.pe -= (double)Fx * (double)rem.x + (double)Fy * (double)rem.y;
   } else {
-    T vx, vy, om;
-    if (MODE == kPrime || (MODE == kBatch && !primed)) {
-      vx = v.x + P.half_dt * ax;
-      vy = v.y + P.half_dt * ay;
-      om = v.z + P.half_dt * al;
-    } else {
-      vx = (v.x + P.half_dt * ax) + P.half_dt * ax;
-      vy = (v.y + P.half_dt * ay) + P.half_dt * ay;
-      om = (v.z + P.half_dt * al) + P.half_dt * al;
-    }
-    T ox, oy;
-    if (sizeof(T) == 4 && P.prem) {
-      float2 r = rem;
-      ox = (T)add_prod_comp((float)p.x, r.x, (float)P.dt, (float)vx);
-      oy = (T)add_prod_comp((float)p.y, r.y, (float)P.dt, (float)vy);
-      B.prem[lp][i] = r;
-    } else {
-      ox = p.x + P.dt * vx;
-      oy = p.y + P.dt * vy;
-    }
-    B.pos[sp ^ 1][i] = V4<T>{ox, oy, p.z, p.w};
-    B.vel[sp ^ 1][i] = V4<T>{vx, vy, om, v.w};
-    L.vmax2 = fmaxf(L.vmax2, (float)(vx * vx + vy * vy));
-    if (!(isfinite(ox) && isfinite(oy) && isfinite(vx) && isfinite(vy) && isfinite(om))) L.bad = true;
+    const Moved<T> m = move_particle<T, MODE>(P, p, v, rem, ax, ay, al, primed, L);
+    if (sizeof(T) == 4 && P.prem) B.prem[lp][i] = m.rem;
+    B.pos[sp ^ 1][i] = m.pos;
+    B.vel[sp ^ 1][i] = m.vel;
   }
 }
 
@@ -1980,7 +2018,13 @@ __global__ void unpack_kernel(Params<T> P, Bufs<T> B, double* pos, double* vel, 
   if (torque) torque[o] = (double)f.z;
 }
 
-static __global__ void set_target_kernel(Ctl* ctl, long long n) { ctl->target = ctl->evals + n; }
+// Start of a step call: the target, and fresh barrier words (a launch whose
+// barrier ran out of time leaves them half used).
+static __global__ void set_target_kernel(Ctl* ctl, long long n) {
+  ctl->target = ctl->evals + n;
+  ctl->epoch = 0u;
+  for (int k = 0; k < 3; ++k) ctl->word[k] = GridWord{0u, 0u, 0u, 0u};
+}
 
 static __global__ void request_rebuild_kernel(Ctl* ctl) { ctl->rebuild_pending = 1; }
 

@@ -1,0 +1,447 @@
+// The resident step kernel (see hm2d_run.cuh).
+#include "hm2d_run.cuh"
+
+namespace tdem {
+namespace hm {
+
+// Grid barrier k = epoch of a cooperative launch of nb blocks, called by every
+// thread; vmax2_bits and bad (shared, or null) hold the block's own values. out
+// (shared) gets {arrivals, largest vmax2_bits, any bad, 1 if the wait ran out}.
+// The words rotate by three: block 0 zeroes the next one before it arrives,
+// when the last waiters of its previous use (two barriers ago) have passed.
+// Waits at most `budget` clocks.
+__device__ __forceinline__ void grid_barrier(Ctl* ctl, unsigned nb, unsigned epoch, const unsigned* block_vmax2,
+                                             const int* block_bad, long long budget, unsigned* out) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned vmax2_bits = block_vmax2 ? *block_vmax2 : 0u;
+    const int bad = block_bad ? *block_bad : 0;
+    GridWord* w = &ctl->word[epoch % 3];
+    if (blockIdx.x == 0) *reinterpret_cast<uint4*>(&ctl->word[(epoch + 1) % 3]) = make_uint4(0u, 0u, 0u, 0u);
+    if (vmax2_bits) atomicMax(&w->vmax2_bits, vmax2_bits);
+    if (bad) atomicOr(&w->bad, 1u);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&w->count) : "memory");
+    const long long start = clock64();
+    unsigned long long lo, hi;
+    unsigned late = 0;
+    while (true) {
+      asm volatile(
+          "{\n\t.reg .b128 t;\n\t"
+          "ld.acquire.gpu.global.b128 t, [%2];\n\t"
+          "mov.b128 {%0, %1}, t;\n\t}"
+          : "=l"(lo), "=l"(hi)
+          : "l"(w)
+          : "memory");
+      if ((unsigned)lo >= nb) break;
+      if (clock64() - start > budget || budget <= 0) {
+        late = 1;
+        atomicOr(&ctl->status, (int)kStatusTimeout);
+        break;
+      }
+    }
+    out[0] = (unsigned)lo;
+    out[1] = (unsigned)(lo >> 32);
+    out[2] = (unsigned)hi;
+    out[3] = late;
+  }
+  __syncthreads();
+}
+
+// Reaction of one evaluation from its per-warp partials {warp, fx, fy} (m of
+// them, distinct warps), summed in warp order by one warp. Returns the sums in
+// lane 0.
+__device__ __forceinline__ void sum_indenter(const double* e, unsigned m, double* sorted, double& sx, double& sy) {
+  const int lane = threadIdx.x & 31;
+  sx = sy = 0.0;
+  for (unsigned a = lane; a < m; a += 32) {
+    const double k0 = e[3 * a];
+    unsigned r = 0;
+    for (unsigned u = 0; u < m; ++u) r += (e[3 * u] < k0) ? 1u : 0u;
+    sorted[2 * r] = e[3 * a + 1];
+    sorted[2 * r + 1] = e[3 * a + 2];
+  }
+  __syncwarp();
+  if (lane == 0) {
+    for (unsigned a = 0; a < m; ++a) {
+      sx += sorted[2 * a];
+      sy += sorted[2 * a + 1];
+    }
+  }
+  __syncwarp();
+}
+
+// Partner state through plain (coherent) loads: the buffers change under a
+// resident launch, so nothing may promise that they are read-only.
+template <class T>
+struct PlainFetch {
+  const V4<T>* pos;
+  const V4<T>* vel;
+  __device__ __forceinline__ V4<T> p(int j) const { return pos[j]; }
+  __device__ __forceinline__ V4<T> v(int j) const { return vel[j]; }
+};
+
+template <class T, bool FEAT, bool LOCAL, bool BIG>
+__global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
+    force_kernel_run(Params<T> P, Bufs<T> B, cudaGraphConditionalHandle h_rebuild, cudaGraphConditionalHandle h_loop,
+                     int use_cond, int pb) {
+  constexpr int MODE = kBatch;  // the first evaluation of a state primes it
+  extern __shared__ __align__(16) unsigned char run_smem[];
+  __shared__ unsigned s_vmax[3], s_out[4];
+  __shared__ int s_bad[3];
+  Ctl* ctl = B.ctl;
+  const int t = threadIdx.x, lane = t & 31;
+  const int n = P.n;
+  const int i = blockIdx.x * pb + t;
+  const bool own = t < pb && i < n;
+  int sp = ctl->sp;
+  const int lp = ctl->lp;
+  long long eval = ctl->evals;
+  const long long target = ctl->target;
+  float disp = ctl->disp;
+  unsigned epoch = ctl->epoch;
+  if (ctl->status & (kStatusNonfinite | kStatusTimeout)) {  // nothing to do with such a state
+    if (blockIdx.x == 0 && t == 0 && (use_cond & 2)) cudaGraphSetConditional(h_loop, 0u);
+    return;
+  }
+  if (t < 3) {
+    s_vmax[t] = 0u;
+    s_bad[t] = 0;
+  }
+  const RunLayout Y = run_layout<T>(P.W, FEAT ? P.BMAX : 0, pb, LOCAL ? 1 : 0, n);
+  V4<T>* const lpos = reinterpret_cast<V4<T>*>(run_smem + Y.pos);
+  V4<T>* const lvel = reinterpret_cast<V4<T>*>(run_smem + Y.vel);
+  V2<T>* const hist = reinterpret_cast<V2<T>*>(run_smem + Y.hist);
+  unsigned* const tail = reinterpret_cast<unsigned*>(run_smem + Y.tail);
+  T* const strain = LOCAL ? reinterpret_cast<T*>(run_smem + Y.strain) : B.strain;
+  // the bond slots of this block's discs, as do_bond addresses them
+  Bufs<T> LB = B;
+  if (FEAT) {
+    LB.bpart[0] = reinterpret_cast<unsigned*>(run_smem + Y.bpart);
+    LB.bref[0] = reinterpret_cast<V2<T>*>(run_smem + Y.bref);
+    LB.bus[0] = reinterpret_cast<V2<T>*>(run_smem + Y.bus);
+    LB.bstr[0] = reinterpret_cast<T*>(run_smem + Y.bstr);
+    LB.bfail[0] = reinterpret_cast<int*>(run_smem + Y.bfail);
+  }
+  // this thread's disc
+  V4<T> p{}, v{}, pi{};
+  uint4 hd = make_uint4(0u, 0u, 0u, 0u);
+  float2 rem = make_float2(0.0f, 0.0f);
+  int bc = 0;
+  if (own) {
+    p = B.pos[sp][i];
+    v = B.vel[sp][i];
+    hd = B.head[lp][i];
+    if (sizeof(T) == 4 && P.prem) rem = B.prem[lp][i];
+    if (LOCAL) {
+      lpos[sp * n + i] = p;
+      lvel[sp * n + i] = v;
+    }
+    const int cnt = (int)(hd.x & 0xFFu);
+    for (int s = kHeadSlots; s < cnt; ++s) tail[(s - kHeadSlots) * pb + t] = B.nbr[lp][(size_t)(s - kHeadSlots) * n + i];
+    for (int s = 0; s < cnt; ++s)
+      if ((hd.x >> (8 + s)) & 1u) hist[s * pb + t] = B.hist[lp][(size_t)s * n + i];
+    if (FEAT && P.BMAX > 0) {
+      bc = B.bcnt[lp][i];
+      pi = B.bpinv[lp][i];
+      for (int u = 0; u < bc; ++u) {
+        const size_t k = (size_t)u * n + i;
+        LB.bpart[0][u * pb + t] = B.bpart[lp][k];
+        LB.bref[0][u * pb + t] = B.bref[lp][k];
+        LB.bus[0][u * pb + t] = B.bus[lp][k];
+        LB.bstr[0][u * pb + t] = B.bstr[lp][k];
+        LB.bfail[0][u * pb + t] = B.bfail[lp][k];
+      }
+    }
+  }
+  const uint4 hd0 = hd;
+  // ledger partials of this warp's 32 discs (slot i / 32), carried in lane 0
+  const size_t gw = (size_t)i >> 5;
+  const bool books = lane == 0 && own;
+  double acc_diss = books ? B.diss_part[gw] : 0.0;
+  double acc_frac = FEAT && books ? B.frac_part[gw] : 0.0;
+  int acc_broke = 0;
+  // The helper warp (one more warp than the discs need, engines with an
+  // indenter) sums the reaction of the evaluation before, in block 0.
+  const bool ind = FEAT && P.irad > T(0);
+  const bool helper = ind && blockIdx.x == 0 && t >= pb;
+  const size_t half = 3 * (size_t)P.ind_slots;
+  double work = 0.0, rx = 0.0, ry = 0.0;
+  auto book_reaction = [&](long long e) {  // evaluation e, helper warp
+    const int par = (int)(e & 1);
+    const unsigned m = *reinterpret_cast<volatile unsigned*>(&ctl->entries[par]);
+    double sx, sy;
+    sum_indenter(B.ind_part + par * half, m, B.ind_part + 2 * half, sx, sy);
+    if (lane == 0) {
+      rx = -sx;
+      ry = -sy;
+      work += (double)P.dt * (sx * P.ind_vx + sy * P.ind_vy);
+      if (e < (long long)P.load_cap) {
+        B.load[2 * e] = -sx;
+        B.load[2 * e + 1] = -sy;
+      }
+      if (m) *reinterpret_cast<volatile unsigned*>(&ctl->entries[par]) = 0u;
+    }
+  };
+  if (helper && lane == 0) work = ctl->tool_work;
+  const long long first = eval;
+  int k3 = 0;  // shared-memory reduction slot of the step
+  bool late = false;
+  unsigned bad = 0u;
+  int rebuild = 0;
+  __syncthreads();
+  while (true) {
+    const int primed = eval > 0 ? 1 : 0;
+    const PlainFetch<T> fetch{LOCAL ? lpos + sp * n : B.pos[sp], LOCAL ? lvel + sp * n : B.vel[sp]};
+    if (FEAT && P.BMAX > 0) {
+      T sv = T(0);
+      if (bc > 0) {
+        T g00 = 0, g01 = 0, g10 = 0, g11 = 0;
+        V4<T> q[kMaxBondSlots];
+#pragma unroll
+        for (int u = 0; u < kMaxBondSlots; ++u)
+          if (u < bc) q[u] = fetch.p((int)(LB.bpart[0][u * pb + t] & kBondIdx));
+#pragma unroll
+        for (int u = 0; u < kMaxBondSlots; ++u) {
+          if (u < bc) {
+            const V2<T> r = LB.bref[0][u * pb + t];
+            const V2<T> cur = cell_delta<T>(P, p, q[u]);
+            const T ux = cur.x - r.x, uy = cur.y - r.y;
+            g00 += ux * r.x;
+            g01 += ux * r.y;
+            g10 += uy * r.x;
+            g11 += uy * r.y;
+          }
+        }
+        sv = shear_invariant<T>(g00, g01, g10, g11, pi);
+      }
+      if (own) strain[i] = sv;
+      if (LOCAL) {
+        __syncthreads();
+      } else {
+        grid_barrier(ctl, gridDim.x, epoch, nullptr, nullptr, P.wait_budget, s_out);
+        ++epoch;
+        if (s_out[3]) {
+          late = true;
+          break;
+        }
+      }
+    }
+    ThreadLedger<T> L;
+    if (own) {
+      Acc<T> fx, fy, tq;
+      if (FEAT && bc > 0) {
+        const T si = strain[i];
+        constexpr int KB = 2;
+#pragma unroll
+        for (int s0 = 0; s0 < kMaxBondSlots; s0 += KB) {
+          if (s0 >= bc) break;
+          BondIn<T> in[KB];
+#pragma unroll
+          for (int u = 0; u < KB; ++u) {
+            if (s0 + u < bc) {
+              const int k = (s0 + u) * pb + t;
+              in[u].w = LB.bpart[0][k];
+              const int j = (int)(in[u].w & kBondIdx);
+              in[u].q = fetch.p(j);
+              in[u].wv = fetch.v(j);
+              in[u].sj = strain[j];
+              in[u].rs = LB.bref[0][k];
+              in[u].us = LB.bus[0][k];
+              in[u].sf = LB.bstr[0][k];
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < KB; ++u)
+            if (s0 + u < bc)
+              do_bond<T, MODE>(P, LB, 0, i, (size_t)((s0 + u) * pb + t), eval, p, v, in[u], si, fx, fy, tq, L, primed);
+        }
+      }
+      const int cnt = (int)(hd.x & 0xFFu);
+      const unsigned mask = hd.x >> 8;
+      unsigned nmask = 0u;
+      // a few candidates at a time: their positions, then the velocities of
+      // those that touch, then the laws in slot order
+      constexpr int KS = BIG ? 1 : kHeadSlots;
+      for (int s0 = 0; s0 < cnt; s0 += KS) {
+        int j[KS];
+        V4<T> q[KS], w[KS];
+        Geo<T> g[KS];
+        bool on[KS];
+#pragma unroll
+        for (int u = 0; u < KS; ++u) {
+          on[u] = s0 + u < cnt;
+          if (on[u]) {
+            const int s = s0 + u;
+            j[u] = (int)(s == 0 ? hd.y : s == 1 ? hd.z : s == 2 ? hd.w : tail[(s - kHeadSlots) * pb + t]);
+            q[u] = fetch.p(j[u]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < KS; ++u) {
+          if (on[u]) {
+            g[u] = slot_geo<T>(P, i, j[u], p, q[u]);
+            on[u] = g[u].d2 < g[u].rs * g[u].rs;
+            if (on[u]) w[u] = fetch.v(j[u]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < KS; ++u) {
+          if (on[u]) {
+            const int s = s0 + u;
+            const bool stored = (mask >> s) & 1u;
+            V2<T>* slot = hist + s * pb + t;
+            const V2<T> xi0 = stored ? *slot : V2<T>{T(0), T(0)};
+            touching_slot<T, MODE>(P, slot, i, j[u], s, g[u], p, v, q[u], w[u], xi0, stored, nmask, fx, fy, tq, L.diss,
+                                   L.un, L.ut, primed);
+          }
+        }
+      }
+      hd.x = (hd.x & 0xFFu) | (nmask << 8);
+      if (FEAT && P.irad > T(0)) indenter_contact<T>(P, eval, p, v, fx, fy, L);
+      wall_contacts<T, MODE>(P, B.whist[lp], i, p, v, fx, fy, tq, L, primed);
+      const T Fx = fx.get(), Fy = fy.get(), Tz = tq.get();
+      const T inv_m = v.w;
+      const bool free = inv_m > T(0);
+      const T inv_i = inv_m * P.kinv / (p.z * p.z);
+      const T ax = free ? Fx * inv_m + P.gx : T(0);
+      const T ay = free ? Fy * inv_m + P.gy : T(0);
+      const T al = Tz * inv_i;
+      const Moved<T> m = move_particle<T, MODE>(P, p, v, rem, ax, ay, al, primed, L);
+      p = m.pos;
+      v = m.vel;
+      rem = m.rem;
+      if (LOCAL) {
+        lpos[(sp ^ 1) * n + i] = p;
+        lvel[(sp ^ 1) * n + i] = v;
+      } else {
+        B.pos[sp ^ 1][i] = p;
+        B.vel[sp ^ 1][i] = v;
+      }
+    } else if (helper && eval > first) {
+      book_reaction(eval - 1);
+    }
+    // the warp's ledger partials (most warps have none)
+    const unsigned wbits = __reduce_max_sync(0xffffffffu, __float_as_uint(L.vmax2));
+    const bool wbad = __any_sync(0xffffffffu, L.bad);
+    if (lane == 0) {
+      if (wbits) atomicMax(&s_vmax[k3], wbits);
+      if (wbad) s_bad[k3] = 1;
+    }
+    if (__any_sync(0xffffffffu, L.diss != T(0))) {
+      T x = L.diss;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+      acc_diss += (double)x;
+    }
+    if (FEAT && __any_sync(0xffffffffu, L.frac != T(0) || L.broke != 0 || L.ifx != T(0) || L.ify != T(0))) {
+      T wf = L.frac, wx = L.ifx, wy = L.ify;
+      int wb = L.broke;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        wf += __shfl_xor_sync(0xffffffffu, wf, off);
+        wx += __shfl_xor_sync(0xffffffffu, wx, off);
+        wy += __shfl_xor_sync(0xffffffffu, wy, off);
+        wb += __shfl_xor_sync(0xffffffffu, wb, off);
+      }
+      acc_frac += (double)wf;
+      acc_broke += wb;
+      if (lane == 0 && (wx != T(0) || wy != T(0))) {
+        const unsigned e = atomicAdd(&ctl->entries[eval & 1], 1u);
+        double* o = B.ind_part + (eval & 1) * half + 3 * (size_t)e;
+        o[0] = (double)gw;
+        o[1] = (double)wx;
+        o[2] = (double)wy;
+      }
+    }
+    const int k1 = k3 == 2 ? 0 : k3 + 1;
+    unsigned vbits;
+    if (t == 0) {  // the next step's slots: last read a step ago
+      s_vmax[k1] = 0u;
+      s_bad[k1] = 0;
+    }
+    if (LOCAL) {
+      __syncthreads();
+      vbits = s_vmax[k3];
+      bad = (unsigned)s_bad[k3];
+    } else {
+      grid_barrier(ctl, gridDim.x, epoch, &s_vmax[k3], &s_bad[k3], P.wait_budget, s_out);
+      ++epoch;
+      if (s_out[3]) {
+        late = true;
+        break;
+      }
+      vbits = s_out[1];
+      bad = s_out[2];
+    }
+    k3 = k1;
+    sp ^= 1;
+    ++eval;
+    disp += sqrtf(__uint_as_float(vbits)) * (float)P.dt;
+    rebuild = disp > P.rebuild_disp ? 1 : 0;
+    if (rebuild || bad || eval >= target) break;
+  }
+  if (late) {  // a barrier ran out of time: the state is not usable
+    if (t == 0 && (use_cond & 2)) cudaGraphSetConditional(h_loop, 0u);
+    return;
+  }
+  // write back what stayed on the chip
+  if (own) {
+    if (LOCAL) {
+      B.pos[sp][i] = p;
+      B.vel[sp][i] = v;
+    }
+    if (sizeof(T) == 4 && P.prem) B.prem[lp][i] = rem;
+    const int cnt = (int)(hd.x & 0xFFu);
+    const unsigned any = (hd.x | hd0.x) >> 8;
+    for (int s = 0; s < cnt; ++s)
+      if ((any >> s) & 1u) B.hist[lp][(size_t)s * n + i] = ((hd.x >> (8 + s)) & 1u) ? hist[s * pb + t] : V2<T>{T(0), T(0)};
+    if (hd.x != hd0.x) B.head[lp][i].x = hd.x;
+    if (FEAT) {
+      for (int u = 0; u < bc; ++u) {
+        const size_t k = (size_t)u * n + i;
+        B.bpart[lp][k] = LB.bpart[0][u * pb + t];
+        B.bus[lp][k] = LB.bus[0][u * pb + t];
+        B.bfail[lp][k] = LB.bfail[0][u * pb + t];
+      }
+      if (P.BMAX > 0 && LOCAL) B.strain[i] = strain[i];
+    }
+  }
+  if (books) {
+    B.diss_part[gw] = acc_diss;
+    if (FEAT) {
+      B.frac_part[gw] = acc_frac;
+      if (acc_broke) atomicAdd(&ctl->broken, acc_broke);
+    }
+  }
+  if (helper) {
+    book_reaction(eval - 1);
+    if (lane == 0) {
+      ctl->reaction_x = rx;
+      ctl->reaction_y = ry;
+      ctl->tool_work = work;
+    }
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    ctl->sp = sp;
+    ctl->evals = eval;
+    ctl->disp = disp;
+    ctl->epoch = epoch;
+    ctl->rebuild_pending = rebuild;
+    if (bad) atomicOr(&ctl->status, (int)kStatusNonfinite);
+    const int keep_going = eval < target && !bad;
+    if (use_cond & 1) cudaGraphSetConditional(h_rebuild, (unsigned)rebuild);
+    if (use_cond & 2) cudaGraphSetConditional(h_loop, (unsigned)keep_going);
+  }
+}
+
+template <class T>
+RunFn<T> run_fn(bool feat, bool local, bool big) {
+  if (local) return feat ? &force_kernel_run<T, true, true, false> : &force_kernel_run<T, false, true, false>;
+  if (big) return feat ? &force_kernel_run<T, true, false, true> : &force_kernel_run<T, false, false, true>;
+  return feat ? &force_kernel_run<T, true, false, false> : &force_kernel_run<T, false, false, false>;
+}
+template RunFn<float> run_fn<float>(bool, bool, bool);
+template RunFn<double> run_fn<double>(bool, bool, bool);
+
+}  // namespace hm
+}  // namespace tdem

@@ -1,0 +1,93 @@
+// Resident step kernel of the single-solve engine: one cooperative launch
+// advances many steps, with a grid barrier in the place of the kernel boundary.
+//
+// What bounds a small or middle-sized engine is not bandwidth but the chain of
+// one step: in the step graph a WHILE iteration costs 3.9 us with an empty
+// body, and a step of 3,249 discs took 11 us. Here each thread owns one disc
+// for the whole launch: its state, list head and remainder stay in registers,
+// its partner indices, contact history and bond slots in shared memory, and
+// only the positions and velocities that partners read go through L2. A grid
+// barrier (one arrival per block, one 16-byte poll that also returns the
+// speed bound and the error flag) costs 1.2 us on 152 blocks. An engine that
+// fits one block keeps the positions in shared memory too and needs only the
+// block's own barrier.
+//
+// Measured (GB300, a pass of upload, n steps, read-back; before -> now):
+// 300 touching discs x 100 steps 1,924 -> 950 us, 3,249 dilute discs x 200
+// steps 2,405 -> 814 us (11 -> 3.4 us a step), 50,071 touching discs x 100
+// steps 1,822 -> 954 us, a 2,328-disc bonded sheet x 200 steps 5,083 -> 2,620
+// us, 65,535 touching discs in FP64 x 50 steps 7,618 -> 6,486 us (bound by the
+// FP64 pipe, not by the chain).
+//
+// The launch ends when the list must be rebuilt, the step target is reached or
+// the state went non-finite; the step graph loops around it. Every disc is
+// evaluated by the same code in the same order as in the one-step kernels, so
+// the states are bit-identical to theirs.
+#pragma once
+
+#include "hm2d_dev.cuh"
+
+namespace tdem {
+namespace hm {
+
+// Threads per block, in two builds: `big` halves the registers of a thread for
+// engines that need every thread of the chip. Without spills the bond, FP64
+// and three-candidates-in-flight code takes up to 255 registers, FP32 contacts
+// 128; the big builds take their candidates one at a time.
+template <class T>
+constexpr int run_block(bool feat, bool big) {
+  return (sizeof(T) == 4 && !feat ? 512 : 256) * (big ? 2 : 1);
+}
+
+// Discs of a block: at least kRunDiscs in a grid; up to kRunLocal (with bonds
+// kRunLocalBonds) stay in one block.
+constexpr int kRunDiscs = 128;
+constexpr int kRunLocal = 512;
+constexpr int kRunLocalBonds = 128;
+
+// Shared memory of a block that owns `pb` discs: byte offsets.
+struct RunLayout {
+  size_t pos, vel, strain, hist, bref, bus, bstr, tail, bpart, bfail, total;
+};
+
+// local: the whole engine (n discs) in one block, positions in shared memory.
+template <class T>
+__host__ __device__ inline RunLayout run_layout(int W, int BM, int pb, int local, int n) {
+  RunLayout L;
+  size_t o = 0;
+  const size_t m = local ? (size_t)n : 0, b = (size_t)pb;
+  L.pos = o;
+  o += 2 * m * sizeof(V4<T>);
+  L.vel = o;
+  o += 2 * m * sizeof(V4<T>);
+  L.hist = o;
+  o += (size_t)W * b * sizeof(V2<T>);
+  L.bref = o;
+  o += (size_t)BM * b * sizeof(V2<T>);
+  L.bus = o;
+  o += (size_t)BM * b * sizeof(V2<T>);
+  L.strain = o;
+  o += (BM > 0 ? m : 0) * sizeof(T);
+  L.bstr = o;
+  o += (size_t)BM * b * sizeof(T);
+  o = (o + 7) & ~size_t(7);
+  L.tail = o;
+  o += (size_t)(W > kHeadSlots ? W - kHeadSlots : 0) * b * 4;
+  L.bpart = o;
+  o += (size_t)BM * b * 4;
+  L.bfail = o;
+  o += (size_t)BM * b * 4;
+  L.total = o;
+  return L;
+}
+
+// The kernel for an engine with (feat) or without bonds or an indenter, in one
+// block with its positions in shared memory (local) or over a cooperative grid
+// (of big blocks).
+template <class T>
+using RunFn = void (*)(Params<T>, Bufs<T>, cudaGraphConditionalHandle, cudaGraphConditionalHandle, int, int);
+template <class T>
+RunFn<T> run_fn(bool feat, bool local, bool big);
+
+}  // namespace hm
+}  // namespace tdem
