@@ -32,7 +32,7 @@
 #include <string>
 #include <vector>
 
-#include "hm2d_dev.cuh"
+#include "batch_run.cuh"
 
 namespace tdem {
 namespace hm {
@@ -638,6 +638,8 @@ struct Batch final : BatchBase {
   int slots = 0;
   int sms = 0;
   int variant = 0;
+  size_t run_smem = 0;
+  bool run_ok = false;  // the resident kernel (variant 0's step loop) can be launched
   bool graph_on = true, graph_failed = false;
   // host view of the instances
   struct Inst {
@@ -792,6 +794,8 @@ struct Batch final : BatchBase {
     int dev = 0;
     TDEM_CUDA_TRY(&err, cudaGetDevice(&dev));
     TDEM_CUDA_TRY(&err, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int rc = plan_run(dev);
+    if (rc) return rc;
     Arena probe;
     carve(probe);
     arena.size = probe.used + 256;
@@ -819,6 +823,26 @@ struct Batch final : BatchBase {
     key_hi = 0;
     return TDEM_OK;
   }
+
+  int plan_run(int dev) {
+    int coop = 0, smem_max = 0, per_sm = 0;
+    TDEM_CUDA_TRY(&err, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    TDEM_CUDA_TRY(&err, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const void* fn = reinterpret_cast<const void*>(batch_run_fn<T>());
+    cudaFuncAttributes at;
+    TDEM_CUDA_TRY(&err, cudaFuncGetAttributes(&at, fn));
+    run_smem = batch_run_smem(G.BMAX, G.prem != 0, sizeof(T) == 4);
+    if (!coop || run_smem + at.sharedSizeBytes > (size_t)smem_max) return TDEM_OK;
+    // the largest any engine asks for (the attribute is the function's, not the engine's)
+    const int most = smem_max - (int)at.sharedSizeBytes;
+    TDEM_CUDA_TRY(&err, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    TDEM_CUDA_TRY(&err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBatchRunBlock<T>, run_smem));
+    run_ok = per_sm >= 1;
+    return TDEM_OK;
+  }
+
+  // The step graph loops around the resident kernel.
+  bool resident() const { return run_ok && variant == 0; }
 
   // Grid of the per-particle / per-key rebuild kernels (grid-stride loops).
   unsigned grid_items(long long items) const {
@@ -865,31 +889,46 @@ struct Batch final : BatchBase {
 
   int add_step_and_rebuild(cudaGraph_t g, cudaGraphConditionalHandle h, cudaGraphConditionalHandle hl) {
     int cond_bits = 3, every = cfg.rebuild_every;
-    void* args[] = {&B, &h, &hl, &cond_bits, &every};
-    const cudaGraphNode_t* dep = nullptr;
-    size_t ndep = 0;
-    cudaGraphNode_t snode;
-    if (G.BMAX > 0) {
-      void* sargs[] = {&G, &B};
-      cudaKernelNodeParams sk = {};
-      sk.func = reinterpret_cast<void*>(&strain_kernel<T, true>);
-      sk.gridDim = dim3(grid_items(cfg.particle_capacity));
-      sk.blockDim = dim3(kThreads);
-      sk.kernelParams = sargs;
-      TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&snode, g, dep, ndep, &sk));
-      dep = &snode;
-      ndep = 1;
-    }
-    cudaKernelNodeParams kp = {};
-    kp.func = reinterpret_cast<void*>(batch_fn<T>(variant, 1));
-    kp.gridDim = dim3(vgrid(variant));
-    kp.blockDim = dim3((unsigned)bvariant_block(variant));
-    kp.kernelParams = args;
-    cudaGraphNode_t pnode;
-    TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&pnode, g, dep, ndep, &kp));
-    kp.func = reinterpret_cast<void*>(batch_fn<T>(variant, 2));
     cudaGraphNode_t knode;
-    TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&knode, g, &pnode, 1, &kp));
+    if (resident()) {
+      int n = G.n, bm = G.BMAX, sl = slots;
+      void* args[] = {&B, &h, &hl, &cond_bits, &every, &n, &bm, &sl};
+      cudaKernelNodeParams kp = {};
+      kp.func = reinterpret_cast<void*>(batch_run_fn<T>());
+      kp.gridDim = dim3((unsigned)sms);
+      kp.blockDim = dim3((unsigned)kBatchRunBlock<T>);
+      kp.sharedMemBytes = (unsigned)run_smem;
+      kp.kernelParams = args;
+      TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&knode, g, nullptr, 0, &kp));
+      cudaKernelNodeAttrValue coop = {};
+      coop.cooperative = 1;
+      TDEM_CUDA_TRY(&err, cudaGraphKernelNodeSetAttribute(knode, cudaLaunchAttributeCooperative, &coop));
+    } else {
+      void* args[] = {&B, &h, &hl, &cond_bits, &every};
+      const cudaGraphNode_t* dep = nullptr;
+      size_t ndep = 0;
+      cudaGraphNode_t snode;
+      if (G.BMAX > 0) {
+        void* sargs[] = {&G, &B};
+        cudaKernelNodeParams sk = {};
+        sk.func = reinterpret_cast<void*>(&strain_kernel<T, true>);
+        sk.gridDim = dim3(grid_items(cfg.particle_capacity));
+        sk.blockDim = dim3(kThreads);
+        sk.kernelParams = sargs;
+        TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&snode, g, dep, ndep, &sk));
+        dep = &snode;
+        ndep = 1;
+      }
+      cudaKernelNodeParams kp = {};
+      kp.func = reinterpret_cast<void*>(batch_fn<T>(variant, 1));
+      kp.gridDim = dim3(vgrid(variant));
+      kp.blockDim = dim3((unsigned)bvariant_block(variant));
+      kp.kernelParams = args;
+      cudaGraphNode_t pnode;
+      TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&pnode, g, dep, ndep, &kp));
+      kp.func = reinterpret_cast<void*>(batch_fn<T>(variant, 2));
+      TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&knode, g, &pnode, 1, &kp));
+    }
     cudaGraphNodeParams ip = {};
     ip.type = cudaGraphNodeTypeConditional;
     ip.conditional.handle = h;
@@ -1141,9 +1180,15 @@ struct Batch final : BatchBase {
   int step(long long n, cudaStream_t s) override {
     int rc = settle(s);  // n == 0 settles admissions and retirements and builds the step graph
     if (rc || n < 0) return rc;
-    if (graph_on && !graph_failed && !exec) {
-      if (build_graph() != TDEM_OK) {
-        graph_failed = true;  // plain launches: the same kernels and results
+    if (graph_on && !graph_failed && !exec && build_graph() != TDEM_OK) {
+      destroy_graphs();
+      cudaGetLastError();
+      // without cooperative nodes the loop takes the one-step kernels, without
+      // conditional graphs steps are plain launches: the same results
+      const bool again = resident();
+      run_ok = false;
+      if (!again || build_graph() != TDEM_OK) {
+        graph_failed = true;
         destroy_graphs();
         cudaGetLastError();
       }
@@ -1161,6 +1206,12 @@ struct Batch final : BatchBase {
     }
     evals += n;
     return TDEM_OK;
+  }
+
+  // After a read of the control block: a grid barrier of the steps ran out of time.
+  int timed_out() {
+    return (host_ctl->status & kStatusTimeout) ? tdem::fail(&err, TDEM_ERR_CUDA, "a bounded grid barrier timed out")
+                                               : TDEM_OK;
   }
 
   int check_id(int id) {
@@ -1201,6 +1252,7 @@ struct Batch final : BatchBase {
     TDEM_CUDA_TRY(&err, cudaMemcpyAsync(host_state, B.istate + id, sizeof(int), cudaMemcpyDeviceToHost, s));
     TDEM_CUDA_TRY(&err, cudaMemcpyAsync(host_ctl, B.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     TDEM_CUDA_TRY(&err, cudaStreamSynchronize(s));
+    if ((rc = timed_out())) return rc;
     if (want_state) {
       if (pos) std::memcpy(pos, stage_host, 2 * m * sizeof(double));
       if (vel) std::memcpy(vel, stage_host + 2 * m, 2 * m * sizeof(double));
@@ -1283,6 +1335,7 @@ struct Batch final : BatchBase {
                                         cudaMemcpyDeviceToHost, s));
     TDEM_CUDA_TRY(&err, cudaMemcpyAsync(host_ctl, B.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     TDEM_CUDA_TRY(&err, cudaStreamSynchronize(s));
+    if ((rc = timed_out())) return rc;
     for (int j = 0; j < count; ++j)
       assemble_ledger(inst[(size_t)ids[j]], all_led_host + (size_t)ids[j] * kInstLedger, all_state_host[ids[j]],
                       out + (size_t)j * TDEM_BATCH_L_COUNT, TDEM_BATCH_L_COUNT);

@@ -463,28 +463,27 @@ __global__ void strain_kernel(Params<T> P, Bufs<T> B) {
 // gathers the current disc's partners and sums its bonds. The same sums in
 // the same order as strain_kernel. Layout [stage][slot][thread].
 constexpr int kStrainBlock = 256;
-constexpr size_t kStrainSmem = (size_t)2 * kStrainBlock * (kMaxBondSlots * (4 + 8) + 16 + 16 + 4);
+constexpr size_t strain_smem_bytes(int block) { return (size_t)2 * block * (kMaxBondSlots * (4 + 8) + 16 + 16 + 4); }
+constexpr size_t kStrainSmem = strain_smem_bytes(kStrainBlock);
 
-template <class T>
-__global__ void __launch_bounds__(kStrainBlock) strain_kernel_async(Params<T> P, Bufs<T> B) {
+template <class T, int BLOCK>
+__device__ __forceinline__ void strain_pass(const Params<T>& P, const Bufs<T>& B, void* smem, int sp, int lp) {
   static_assert(sizeof(T) == 4, "the pipelined strain serves FP32 engines");
   using bulk::cp16;
   using bulk::cp4;
   using bulk::cp8;
   using bulk::cp_commit;
   using bulk::cp_wait;
-  constexpr int BL = kStrainBlock, S = kMaxBondSlots;
-  extern __shared__ uint4 strain_smem[];
-  V4<T>* spos = reinterpret_cast<V4<T>*>(strain_smem);              // [2][BL]
+  constexpr int BL = BLOCK, S = kMaxBondSlots;
+  V4<T>* spos = reinterpret_cast<V4<T>*>(smem);              // [2][BL]
   V4<T>* spi = spos + 2 * BL;                                        // [2][BL]
   V2<T>* sref = reinterpret_cast<V2<T>*>(spi + 2 * BL);              // [2][S][BL]
   unsigned* sw = reinterpret_cast<unsigned*>(sref + 2 * S * BL);     // [2][S][BL]
   int* sbc = reinterpret_cast<int*>(sw + 2 * S * BL);                // [2][BL]
-  const int sp = B.ctl->sp, lp = B.ctl->lp;
   const int n = P.n, BM = P.BMAX;
   const int t = threadIdx.x;
   const int stride = gridDim.x * BL;
-  const V4<T>* __restrict__ pos = B.pos[sp];
+  const V4<T>* pos = B.pos[sp];
   const unsigned* __restrict__ bpart = B.bpart[lp];
   const V2<T>* __restrict__ bref = B.bref[lp];
   auto stage = [&](int i, int st) {
@@ -532,6 +531,12 @@ __global__ void __launch_bounds__(kStrainBlock) strain_kernel_async(Params<T> P,
     B.strain[i] = sv;
   }
   cp_wait<0>();
+}
+
+template <class T>
+__global__ void __launch_bounds__(kStrainBlock) strain_kernel_async(Params<T> P, Bufs<T> B) {
+  extern __shared__ uint4 strain_smem[];
+  strain_pass<T, kStrainBlock>(P, B, strain_smem, B.ctl->sp, B.ctl->lp);
 }
 
 // Per-thread ledger terms of the particles a thread processed.
@@ -1262,38 +1267,31 @@ constexpr size_t async_smem(int block, bool prem) {
 // are staged with its own state, one disc ahead, into [2][BMAX][BLOCK] words,
 // [2][BLOCK] counts and [2][BLOCK] strains after the records above, so the
 // bond partners' gathers start without a dependent load.
-template <class T, int MODE, int BLOCK, int MINB, bool FEAT, bool WMAJ = false, bool PW = false>
-__global__ void __launch_bounds__(BLOCK, MINB) force_kernel_async(Params<T> P, Bufs<T> B,
-                                                                  cudaGraphConditionalHandle h_rebuild,
-                                                                  cudaGraphConditionalHandle h_loop, int use_cond,
-                                                                  int primed, StepHint hint) {
+template <class T, int MODE, int BLOCK, bool FEAT, bool WMAJ, bool PW, class F, class D>
+__device__ __forceinline__ void async_pass(const Params<T>& P, const Bufs<T>& B, const F& fetch, uint4* smem, int sp,
+                                           int lp, int primed, long long eval, ThreadLedger<T>& L, D disc_done) {
   static_assert(MODE != kPeek, "read-back uses force_kernel");
   static_assert(sizeof(V4<T>) == 16, "one 16-byte copy per record");
   using bulk::cp16;
   using bulk::cp8;
   using bulk::cp_commit;
   using bulk::cp_wait;
-  extern __shared__ uint4 async_smem_base[];
-  const StepCtl c = load_step_ctl(B.ctl, hint);
-  const int sp = c.sp, lp = c.lp;
   const int t = threadIdx.x;
   const int end = P.n;
   const int stride = gridDim.x * BLOCK;
-  uint4* sh = async_smem_base;                                           // [3][BLOCK]
-  V4<T>* spos = reinterpret_cast<V4<T>*>(async_smem_base + 3 * BLOCK);  // [2][BLOCK]
+  uint4* sh = smem;                                        // [3][BLOCK]
+  V4<T>* spos = reinterpret_cast<V4<T>*>(smem + 3 * BLOCK);  // [2][BLOCK]
   V4<T>* svel = spos + 2 * BLOCK;                                        // [2][BLOCK]
   V4<T>* sq = svel + 2 * BLOCK;                                          // [2][3][BLOCK]
   float2* srem = reinterpret_cast<float2*>(sq + 6 * BLOCK);              // [2][BLOCK]
   const bool pr = P.prem != 0;
-  const float2* __restrict__ prem = B.prem[lp];
-  const V4<T>* __restrict__ pos = B.pos[sp];
-  const V4<T>* __restrict__ vel = B.vel[sp];
-  const uint4* __restrict__ head = B.head[lp];
-  const GlobalFetch<T> fetch{pos, vel};
-  ThreadLedger<T> L;
+  const float2* prem = B.prem[lp];
+  const auto pos = fetch.pos;
+  const auto vel = fetch.vel;
+  const uint4* head = B.head[lp];
   // bond staging (PW): slot words, counts and strains of the disc in flight
   const int BM = (PW && FEAT) ? P.BMAX : 0;
-  unsigned* sbw = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(async_smem_base) +
+  unsigned* sbw = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(smem) +
                                               (size_t)kAsyncRecords * BLOCK * 16 + (pr ? (size_t)2 * BLOCK * 8 : 0));
   int* sbc = reinterpret_cast<int*>(sbw + 2 * BM * BLOCK);
   T* ssi = reinterpret_cast<T*>(sbc + 2 * BLOCK);
@@ -1372,16 +1370,29 @@ __global__ void __launch_bounds__(BLOCK, MINB) force_kernel_async(Params<T> P, B
     if (cnt > 2) q2 = q[2 * BLOCK];
     const float2 rm = pr ? srem[s * BLOCK + t] : make_float2(0.0f, 0.0f);
     if constexpr (PW && FEAT) {
-      process_particle_q<T, MODE, FEAT, GlobalFetch<T>, false, true>(
-          P, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, primed, c.evals, L, &rm, sbw + s * BM * BLOCK + t, BLOCK,
+      process_particle_q<T, MODE, FEAT, F, false, true>(
+          P, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, primed, eval, L, &rm, sbw + s * BM * BLOCK + t, BLOCK,
           BM > 0 ? sbc[s * BLOCK + t] : 0, BM > 0 ? ssi[s * BLOCK + t] : T(0));
     } else {
-      process_particle_q<T, MODE, FEAT>(P, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, primed, c.evals, L, &rm);
+      process_particle_q<T, MODE, FEAT, F>(P, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, primed, eval, L, &rm);
     }
+    disc_done(i);
     h0 = h1;
     s ^= 1;
   }
   cp_wait<0>();
+}
+
+template <class T, int MODE, int BLOCK, int MINB, bool FEAT, bool WMAJ = false, bool PW = false>
+__global__ void __launch_bounds__(BLOCK, MINB) force_kernel_async(Params<T> P, Bufs<T> B,
+                                                                  cudaGraphConditionalHandle h_rebuild,
+                                                                  cudaGraphConditionalHandle h_loop, int use_cond,
+                                                                  int primed, StepHint hint) {
+  extern __shared__ uint4 async_smem_base[];
+  const StepCtl c = load_step_ctl(B.ctl, hint);
+  ThreadLedger<T> L;
+  const GlobalFetch<T> fetch{B.pos[c.sp], B.vel[c.sp]};
+  async_pass<T, MODE, BLOCK, FEAT, WMAJ, PW>(P, B, fetch, async_smem_base, c.sp, c.lp, primed, c.evals, L, [](int) {});
   commit_epilogue<T, FEAT>(P, B, c, L, h_rebuild, h_loop, use_cond);
 }
 

@@ -4,49 +4,6 @@
 namespace tdem {
 namespace hm {
 
-// Grid barrier k = epoch of a cooperative launch of nb blocks, called by every
-// thread; vmax2_bits and bad (shared, or null) hold the block's own values. out
-// (shared) gets {arrivals, largest vmax2_bits, any bad, 1 if the wait ran out}.
-// The words rotate by three: block 0 zeroes the next one before it arrives,
-// when the last waiters of its previous use (two barriers ago) have passed.
-// Waits at most `budget` clocks.
-__device__ __forceinline__ void grid_barrier(Ctl* ctl, unsigned nb, unsigned epoch, const unsigned* block_vmax2,
-                                             const int* block_bad, long long budget, unsigned* out) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned vmax2_bits = block_vmax2 ? *block_vmax2 : 0u;
-    const int bad = block_bad ? *block_bad : 0;
-    GridWord* w = &ctl->word[epoch % 3];
-    if (blockIdx.x == 0) *reinterpret_cast<uint4*>(&ctl->word[(epoch + 1) % 3]) = make_uint4(0u, 0u, 0u, 0u);
-    if (vmax2_bits) atomicMax(&w->vmax2_bits, vmax2_bits);
-    if (bad) atomicOr(&w->bad, 1u);
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&w->count) : "memory");
-    const long long start = clock64();
-    unsigned long long lo, hi;
-    unsigned late = 0;
-    while (true) {
-      asm volatile(
-          "{\n\t.reg .b128 t;\n\t"
-          "ld.acquire.gpu.global.b128 t, [%2];\n\t"
-          "mov.b128 {%0, %1}, t;\n\t}"
-          : "=l"(lo), "=l"(hi)
-          : "l"(w)
-          : "memory");
-      if ((unsigned)lo >= nb) break;
-      if (clock64() - start > budget || budget <= 0) {
-        late = 1;
-        atomicOr(&ctl->status, (int)kStatusTimeout);
-        break;
-      }
-    }
-    out[0] = (unsigned)lo;
-    out[1] = (unsigned)(lo >> 32);
-    out[2] = (unsigned)hi;
-    out[3] = late;
-  }
-  __syncthreads();
-}
-
 // Reaction of one evaluation from its per-warp partials {warp, fx, fy} (m of
 // them, distinct warps), summed in warp order by one warp. Returns the sums in
 // lane 0.
@@ -70,15 +27,31 @@ __device__ __forceinline__ void sum_indenter(const double* e, unsigned m, double
   __syncwarp();
 }
 
-// Partner state through plain (coherent) loads: the buffers change under a
-// resident launch, so nothing may promise that they are read-only.
-template <class T>
-struct PlainFetch {
-  const V4<T>* pos;
-  const V4<T>* vel;
-  __device__ __forceinline__ V4<T> p(int j) const { return pos[j]; }
-  __device__ __forceinline__ V4<T> v(int j) const { return vel[j]; }
+// The indenter's running totals, in lane 0 of the warp that books them.
+struct Reaction {
+  double work, x, y;
 };
+
+// Reaction of evaluation e from its partials (entries[e & 1] of them), by one
+// warp, after the evaluation's barrier; the count is cleared for evaluation
+// e + 2, whose first partials come after the next barrier.
+template <class T>
+__device__ __forceinline__ void book_reaction(const Params<T>& P, const Bufs<T>& B, long long e, size_t half,
+                                              Reaction& R) {
+  const int par = (int)(e & 1);
+  const unsigned m = *reinterpret_cast<volatile unsigned*>(&B.ctl->entries[par]);
+  double sx, sy;
+  sum_indenter(B.ind_part + par * half, m, B.ind_part + 2 * half, sx, sy);
+  if ((threadIdx.x & 31) != 0) return;
+  R.x = -sx;
+  R.y = -sy;
+  R.work += (double)P.dt * (sx * P.ind_vx + sy * P.ind_vy);
+  if (e < (long long)P.load_cap) {
+    B.load[2 * e] = -sx;
+    B.load[2 * e + 1] = -sy;
+  }
+  if (m) *reinterpret_cast<volatile unsigned*>(&B.ctl->entries[par]) = 0u;
+}
 
 template <class T, bool FEAT, bool LOCAL, bool BIG>
 __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
@@ -165,24 +138,8 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
   const bool ind = FEAT && P.irad > T(0);
   const bool helper = ind && blockIdx.x == 0 && t >= pb;
   const size_t half = 3 * (size_t)P.ind_slots;
-  double work = 0.0, rx = 0.0, ry = 0.0;
-  auto book_reaction = [&](long long e) {  // evaluation e, helper warp
-    const int par = (int)(e & 1);
-    const unsigned m = *reinterpret_cast<volatile unsigned*>(&ctl->entries[par]);
-    double sx, sy;
-    sum_indenter(B.ind_part + par * half, m, B.ind_part + 2 * half, sx, sy);
-    if (lane == 0) {
-      rx = -sx;
-      ry = -sy;
-      work += (double)P.dt * (sx * P.ind_vx + sy * P.ind_vy);
-      if (e < (long long)P.load_cap) {
-        B.load[2 * e] = -sx;
-        B.load[2 * e + 1] = -sy;
-      }
-      if (m) *reinterpret_cast<volatile unsigned*>(&ctl->entries[par]) = 0u;
-    }
-  };
-  if (helper && lane == 0) work = ctl->tool_work;
+  Reaction R{0.0, 0.0, 0.0};
+  if (helper && lane == 0) R.work = ctl->tool_work;
   const long long first = eval;
   int k3 = 0;  // shared-memory reduction slot of the step
   bool late = false;
@@ -318,7 +275,7 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
         B.vel[sp ^ 1][i] = v;
       }
     } else if (helper && eval > first) {
-      book_reaction(eval - 1);
+      book_reaction(P, B, eval - 1, half, R);
     }
     // the warp's ledger partials (most warps have none)
     const unsigned wbits = __reduce_max_sync(0xffffffffu, __float_as_uint(L.vmax2));
@@ -414,11 +371,11 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
     }
   }
   if (helper) {
-    book_reaction(eval - 1);
+    book_reaction(P, B, eval - 1, half, R);
     if (lane == 0) {
-      ctl->reaction_x = rx;
-      ctl->reaction_y = ry;
-      ctl->tool_work = work;
+      ctl->reaction_x = R.x;
+      ctl->reaction_y = R.y;
+      ctl->tool_work = R.work;
     }
   }
   if (blockIdx.x == 0 && t == 0) {

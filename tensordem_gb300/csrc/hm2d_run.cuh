@@ -30,6 +30,59 @@
 namespace tdem {
 namespace hm {
 
+// Grid barrier k = epoch of a cooperative launch of nb blocks, called by every
+// thread; vmax2_bits and bad (shared, or null) hold the block's own values. out
+// (shared) gets {arrivals, largest vmax2_bits, any bad, 1 if the wait ran out}.
+// The words rotate by three: block 0 zeroes the next one before it arrives,
+// when the last waiters of its previous use (two barriers ago) have passed.
+// Waits at most `budget` clocks.
+__device__ __forceinline__ void grid_barrier(Ctl* ctl, unsigned nb, unsigned epoch, const unsigned* block_vmax2,
+                                             const int* block_bad, long long budget, unsigned* out) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned vmax2_bits = block_vmax2 ? *block_vmax2 : 0u;
+    const int bad = block_bad ? *block_bad : 0;
+    GridWord* w = &ctl->word[epoch % 3];
+    if (blockIdx.x == 0) *reinterpret_cast<uint4*>(&ctl->word[(epoch + 1) % 3]) = make_uint4(0u, 0u, 0u, 0u);
+    if (vmax2_bits) atomicMax(&w->vmax2_bits, vmax2_bits);
+    if (bad) atomicOr(&w->bad, 1u);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&w->count) : "memory");
+    const long long start = clock64();
+    unsigned long long lo, hi;
+    unsigned late = 0;
+    while (true) {
+      asm volatile(
+          "{\n\t.reg .b128 t;\n\t"
+          "ld.acquire.gpu.global.b128 t, [%2];\n\t"
+          "mov.b128 {%0, %1}, t;\n\t}"
+          : "=l"(lo), "=l"(hi)
+          : "l"(w)
+          : "memory");
+      if ((unsigned)lo >= nb) break;
+      if (clock64() - start > budget || budget <= 0) {
+        late = 1;
+        atomicOr(&ctl->status, (int)kStatusTimeout);
+        break;
+      }
+    }
+    out[0] = (unsigned)lo;
+    out[1] = (unsigned)(lo >> 32);
+    out[2] = (unsigned)hi;
+    out[3] = late;
+  }
+  __syncthreads();
+}
+
+// Partner state through plain (coherent) loads: the buffers change under a
+// resident launch, so nothing may promise that they are read-only.
+template <class T>
+struct PlainFetch {
+  const V4<T>* pos;
+  const V4<T>* vel;
+  __device__ __forceinline__ V4<T> p(int j) const { return pos[j]; }
+  __device__ __forceinline__ V4<T> v(int j) const { return vel[j]; }
+};
+
 // Threads per block, in two builds: `big` halves the registers of a thread for
 // engines that need every thread of the chip. Without spills the bond, FP64
 // and three-candidates-in-flight code takes up to 255 registers, FP32 contacts
