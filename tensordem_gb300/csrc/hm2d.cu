@@ -318,10 +318,14 @@ struct Engine final : EngineBase {
   int vgrid[kVariants] = {};
   int nwarp_slots = 0;
   int sgrid = 1;  // grid of the pipelined strain kernel (FP32 engines with bonds)
-  // resident step kernel (variant 0's step loop): discs per block, grid, build
-  RunFn<T> run = nullptr;
-  int run_pb = 0, run_grid = 0, run_threads = 0;
-  size_t run_smem = 0;
+  // resident step kernels: the default loop's (variant 0) and the pipelined
+  // one of variant 10 or 11
+  struct RunPlan {
+    RunFn<T> fn = nullptr;
+    int pb = 0, grid = 0, threads = 0;  // discs per block (one per thread), blocks, threads
+    size_t smem = 0;
+  };
+  RunPlan run0, runp;
   bool primed = false;
   bool has_state = false;
   bool graph_on = true;
@@ -495,18 +499,34 @@ struct Engine final : EngineBase {
       TDEM_CUDA_TRY(&err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn),
                                                                         pb + extra, smem));
       if (per_sm < 1) continue;
-      run = fn;
-      run_pb = pb;
-      run_grid = (P.n + pb - 1) / pb;
-      run_threads = pb + extra;
-      run_smem = smem;
+      run0 = RunPlan{fn, pb, (P.n + pb - 1) / pb, pb + extra, smem};
       break;
+    }
+    if constexpr (sizeof(T) == 4) {
+      const int v = f ? kAsyncHalfVariant : kAsyncWideVariant + 1;
+      const int block = f ? kRunAsync<true> : kRunAsync<false>;
+      const size_t smem = std::max(smem_of(v), f && P.BMAX > 0 ? strain_smem_bytes(block) : size_t(0));
+      for (bool chunked : {false, true}) {
+        if (chunked && run0.fn) break;  // one disc per thread is faster
+        RunFn<T> fn = run_async_fn(f, chunked);
+        int per_sm = 0;
+        TDEM_CUDA_TRY(&err, cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+        TDEM_CUDA_TRY(&err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn),
+                                                                          block, smem));
+        if (per_sm < 1) continue;
+        (chunked ? run0 : runp) = RunPlan{fn, 0, std::min((P.n + block - 1) / block, sms), block, smem};
+      }
     }
     return TDEM_OK;
   }
 
-  // The step graph loops around the resident kernel.
-  bool resident() const { return run && variant == 0; }
+  // The resident kernel that the step graph loops around, if the variant has one.
+  const RunPlan* resident() const {
+    if (variant == 0) return run0.fn ? &run0 : nullptr;
+    if (variant == (feat() ? kAsyncHalfVariant : kAsyncWideVariant + 1)) return runp.fn ? &runp : nullptr;
+    return nullptr;
+  }
 
   bool feat() const { return P.BMAX > 0 || P.irad > T(0); }
   // launch shape of a variant's step kernel (the FP64-sum form has one shape)
@@ -566,13 +586,14 @@ struct Engine final : EngineBase {
   int add_step_and_rebuild(cudaGraph_t g, const cudaGraphNode_t* dep, size_t ndep,
                            cudaGraphConditionalHandle h, cudaGraphConditionalHandle hl, int cond_bits) {
     cudaGraphNode_t knode;
-    if (resident()) {
-      void* args[] = {&P, &B, &h, &hl, &cond_bits, &run_pb};
+    if (const RunPlan* r = resident()) {
+      int discs = r->pb;
+      void* args[] = {&P, &B, &h, &hl, &cond_bits, &discs};
       cudaKernelNodeParams kp = {};
-      kp.func = reinterpret_cast<void*>(run);
-      kp.gridDim = dim3((unsigned)run_grid);
-      kp.blockDim = dim3((unsigned)run_threads);
-      kp.sharedMemBytes = (unsigned)run_smem;
+      kp.func = reinterpret_cast<void*>(r->fn);
+      kp.gridDim = dim3((unsigned)r->grid);
+      kp.blockDim = dim3((unsigned)r->threads);
+      kp.sharedMemBytes = (unsigned)r->smem;
       kp.kernelParams = args;
       TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&knode, g, dep, ndep, &kp));
       cudaKernelNodeAttrValue coop = {};
@@ -669,7 +690,7 @@ struct Engine final : EngineBase {
     if (build_graph() == TDEM_OK) return;
     destroy_graphs();
     if (resident()) {
-      run = nullptr;
+      run0.fn = runp.fn = nullptr;
       cudaGetLastError();
       if (build_graph() == TDEM_OK) return;
       destroy_graphs();

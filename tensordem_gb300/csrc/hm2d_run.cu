@@ -391,6 +391,167 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
   }
 }
 
+// Resident form of the pipelined step (FP32), for engines of many discs per
+// thread: the one-step kernel's pass over the discs, with a grid barrier in the
+// place of the launch. At 1,048,576 discs the launch, its ramp and its last
+// block cost 6 us of a 24 us step. Measured (GB300, steps and a state read):
+// 1,048,576 discs x 100 steps 2,894 -> 2,717 us, 4,194,304 discs x 40 steps
+// 6,708 -> 4,920 us (the default loop had been the one-thread-per-disc kernel),
+// the 1,048,576-disc bonded sheet x 40 steps 6,026 -> 5,605 us.
+// CHUNKED: ledger partials per 32 sorted discs, as variant 0 books them; else
+// per warp of the grid, as the pipelined variants do.
+template <class T, int BLOCK, bool FEAT, bool CHUNKED>
+__global__ void __launch_bounds__(BLOCK, 1)
+    force_kernel_run_async(Params<T> P, Bufs<T> B, cudaGraphConditionalHandle h_rebuild,
+                           cudaGraphConditionalHandle h_loop, int use_cond, int) {
+  extern __shared__ __align__(16) unsigned char run_smem[];
+  __shared__ unsigned s_vmax[3], s_out[4];
+  __shared__ int s_bad[3];
+  Ctl* ctl = B.ctl;
+  const int t = threadIdx.x, lane = t & 31;
+  int sp = ctl->sp;
+  const int lp = ctl->lp;
+  long long eval = ctl->evals;
+  const long long target = ctl->target, first = eval;
+  float disp = ctl->disp;
+  unsigned epoch = ctl->epoch;
+  if (ctl->status & (kStatusNonfinite | kStatusTimeout)) {
+    if (blockIdx.x == 0 && t == 0 && (use_cond & 2)) cudaGraphSetConditional(h_loop, 0u);
+    return;
+  }
+  if (t < 3) {
+    s_vmax[t] = 0u;
+    s_bad[t] = 0;
+  }
+  const size_t warp = (size_t)blockIdx.x * (BLOCK / 32) + (t >> 5);
+  double acc_diss = 0.0, acc_frac = 0.0;
+  int acc_broke = 0;
+  if (!CHUNKED && lane == 0) {
+    acc_diss = B.diss_part[warp];
+    if (FEAT) acc_frac = B.frac_part[warp];
+  }
+  const size_t half = 3 * (size_t)P.ind_slots;
+  // block 0's first warp sums the reaction of the evaluation before
+  const bool books = FEAT && P.irad > T(0) && blockIdx.x == 0 && t < 32;
+  Reaction R{books && lane == 0 ? ctl->tool_work : 0.0, 0.0, 0.0};
+  int k3 = 0, rebuild = 0;
+  unsigned bad = 0u;
+  bool late = false;
+  __syncthreads();
+  while (true) {
+    if (FEAT && books && eval > first) book_reaction(P, B, eval - 1, half, R);
+    if (FEAT && P.BMAX > 0) {
+      strain_pass<T, BLOCK>(P, B, run_smem, sp, lp);
+      grid_barrier(ctl, gridDim.x, epoch++, nullptr, nullptr, P.wait_budget, s_out);
+      if (s_out[3]) {
+        late = true;
+        break;
+      }
+    }
+    ThreadLedger<T> L;
+    const PlainFetch<T> fetch{B.pos[sp], B.vel[sp]};
+    // one ledger slot: the terms of `count` lanes (the last chunk may be short)
+    auto book = [&](unsigned m, int count, size_t slot) {
+      auto total = [&](auto x) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+          const auto y = __shfl_xor_sync(m, x, off);
+          x += (lane ^ off) < count ? y : decltype(x)(0);
+        }
+        return x;
+      };
+      if (__any_sync(m, L.diss != T(0))) {
+        const T x = total(L.diss);
+        if (CHUNKED) {
+          if (lane == 0) atomicAdd(&B.diss_part[slot], (double)x);
+        } else {
+          acc_diss += (double)x;
+        }
+      }
+      if (FEAT && __any_sync(m, L.frac != T(0) || L.broke != 0 || L.ifx != T(0) || L.ify != T(0))) {
+        const T f = total(L.frac), x = total(L.ifx), y = total(L.ify);
+        const int broke = total(L.broke);
+        if (CHUNKED) {
+          if (lane == 0 && f != T(0)) atomicAdd(&B.frac_part[slot], (double)f);
+        } else {
+          acc_frac += (double)f;
+        }
+        acc_broke += broke;
+        if (lane == 0 && (x != T(0) || y != T(0))) {
+          const unsigned e = atomicAdd(&ctl->entries[eval & 1], 1u);
+          double* o = B.ind_part + (eval & 1) * half + 3 * (size_t)e;
+          o[0] = (double)slot;
+          o[1] = (double)x;
+          o[2] = (double)y;
+        }
+      }
+    };
+    async_pass<T, kBatch, BLOCK, FEAT, true, FEAT>(
+        P, B, fetch, reinterpret_cast<uint4*>(run_smem), sp, lp, eval > 0 ? 1 : 0, eval, L, [&](int i) {
+          if (CHUNKED) {
+            const int count = min(32, P.n - (i - lane));
+            book(count == 32 ? 0xffffffffu : (1u << count) - 1u, count, (size_t)i >> 5);
+            L.diss = L.frac = L.ifx = L.ify = T(0);
+            L.broke = 0;
+          }
+        });
+    __syncwarp();
+    if (!CHUNKED) book(0xffffffffu, 32, warp);
+    const unsigned wbits = __reduce_max_sync(0xffffffffu, __float_as_uint(L.vmax2));
+    const bool wbad = __any_sync(0xffffffffu, L.bad);
+    if (lane == 0) {
+      if (wbits) atomicMax(&s_vmax[k3], wbits);
+      if (wbad) s_bad[k3] = 1;
+    }
+    const int k1 = k3 == 2 ? 0 : k3 + 1;
+    if (t == 0) {
+      s_vmax[k1] = 0u;
+      s_bad[k1] = 0;
+    }
+    grid_barrier(ctl, gridDim.x, epoch++, &s_vmax[k3], &s_bad[k3], P.wait_budget, s_out);
+    if (s_out[3]) {
+      late = true;
+      break;
+    }
+    bad = s_out[2];
+    k3 = k1;
+    sp ^= 1;
+    ++eval;
+    disp += sqrtf(__uint_as_float(s_out[1])) * (float)P.dt;
+    rebuild = disp > P.rebuild_disp ? 1 : 0;
+    if (rebuild || bad || eval >= target) break;
+  }
+  if (late) {
+    if (t == 0 && (use_cond & 2)) cudaGraphSetConditional(h_loop, 0u);
+    return;
+  }
+  if (lane == 0) {
+    if (!CHUNKED) {
+      B.diss_part[warp] = acc_diss;
+      if (FEAT) B.frac_part[warp] = acc_frac;
+    }
+    if (FEAT && acc_broke) atomicAdd(&ctl->broken, acc_broke);
+  }
+  if (FEAT && books) {
+    book_reaction(P, B, eval - 1, half, R);
+    if (lane == 0) {
+      ctl->reaction_x = R.x;
+      ctl->reaction_y = R.y;
+      ctl->tool_work = R.work;
+    }
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    ctl->sp = sp;
+    ctl->evals = eval;
+    ctl->disp = disp;
+    ctl->epoch = epoch;
+    ctl->rebuild_pending = rebuild;
+    if (bad) atomicOr(&ctl->status, (int)kStatusNonfinite);
+    if (use_cond & 1) cudaGraphSetConditional(h_rebuild, (unsigned)rebuild);
+    if (use_cond & 2) cudaGraphSetConditional(h_loop, (unsigned)(eval < target && !bad ? 1 : 0));
+  }
+}
+
 template <class T>
 RunFn<T> run_fn(bool feat, bool local, bool big) {
   if (local) return feat ? &force_kernel_run<T, true, true, false> : &force_kernel_run<T, false, true, false>;
@@ -399,6 +560,12 @@ RunFn<T> run_fn(bool feat, bool local, bool big) {
 }
 template RunFn<float> run_fn<float>(bool, bool, bool);
 template RunFn<double> run_fn<double>(bool, bool, bool);
+
+RunFn<float> run_async_fn(bool feat, bool chunked) {
+  constexpr int W = kRunAsync<false>, H = kRunAsync<true>;
+  if (feat) return chunked ? &force_kernel_run_async<float, H, true, true> : &force_kernel_run_async<float, H, true, false>;
+  return chunked ? &force_kernel_run_async<float, W, false, true> : &force_kernel_run_async<float, W, false, false>;
+}
 
 }  // namespace hm
 }  // namespace tdem

@@ -142,5 +142,11 @@ using RunFn = void (*)(Params<T>, Bufs<T>, cudaGraphConditionalHandle, cudaGraph
 template <class T>
 RunFn<T> run_fn(bool feat, bool local, bool big);
 
+// The pipelined form for FP32 engines of many discs per thread, in the block
+// shapes of variants 10 (without bonds or indenter) and 11 (with).
+template <bool FEAT>
+constexpr int kRunAsync = FEAT ? 512 : 1024;
+RunFn<float> run_async_fn(bool feat, bool chunked);
+
 }  // namespace hm
 }  // namespace tdem
