@@ -1,11 +1,11 @@
 // Reference-mode engine: the FP64 2-D bonded-disc step of the reference's
 // IceDEM (src/tensordem/dem.py), on sm_103a.
 //
-// Design. One CTA owns one instance and runs many steps per launch; the
-// instance's positions, velocities, per-disc shear strain and forces sit in
-// shared memory between the phases of a step, so a step costs no global
-// round trip beyond the caller-owned state writes. Each disc's force is
-// accumulated by one thread in exactly the order of the reference's two
+// Design. One thread-block cluster (one CTA for discs of more than eight
+// bonds) owns one instance and runs many steps per launch; the instance's
+// positions, velocities, per-disc shear strain and forces sit in shared memory
+// between the phases of a step, so a step costs no global round trip. Each
+// disc's force is summed in exactly the order of the reference's two
 // index_add_ calls (dem.py:290-292): partners j > k ascending (disc k is the
 // pair's i), then partners i < k ascending (disc k is the pair's j). Pairs
 // that are neither alive bonds nor overlapping contribute +-0 in the
@@ -17,6 +17,7 @@
 // operation is torch's CPU vector_norm, which sums the squares of a 2-vector
 // as fma(y, y, x*x); distances are computed that way, with fma() explicitly.
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -265,7 +266,643 @@ __global__ void __launch_bounds__(512) icedem_fragment_kernel(Params P, Topo T, 
 }
 
 // ---------------------------------------------------------------------------
-// The fused step kernel. mode 0: n_steps full steps; mode 1: one force
+// The step over a thread-block cluster.
+//
+// One SM executes two FP64 lanes a clock, so the 1,900 FP64 warp instructions of
+// a 105-disc step take 15 us on one SM however they are arranged, and the
+// one-thread-per-disc kernel below took 66 us. Here the discs are dealt to the
+// CTAs of one cluster. A group of eight lanes serves a disc, one lane per bond:
+// each lane forms its bond's terms and only the sums the reference orders run
+// in order (the four components of the shear sum on four lanes, the two of the
+// force on two). Every CTA keeps all positions, velocities and shear strains in
+// its shared memory; the owner of a disc writes them to every CTA (distributed
+// shared memory). Two cluster barriers separate the phases of a step (three
+// when the positions do not fit twice). A ledger warp per CTA sums the terms
+// of the step before, one lane per term, while the others compute.
+//
+// The order of every force sum is the reference's: partners above the disc
+// ascending, then partners below it. The alive bonds and the near pairs found
+// by the FP32 scan get their places in that order from the scan's ballots.
+//
+// Measured (GB300): the 21 x 5 demonstration from its first state, 250 steps,
+// one force evaluation: 16,514 -> 3,217 us (66 -> 12 us a step).
+// ---------------------------------------------------------------------------
+constexpr int kGroup = 8;         // lanes of a disc: the lattice's bonds per disc
+constexpr int kClusterWarps = 15;  // compute warps of a CTA at most (and one ledger warp)
+constexpr int kList = 32;         // force terms of one disc held in shared memory
+constexpr int kAcc = 16;          // per-disc ledger terms
+constexpr int kMaxCluster = 16;
+
+// Shared memory of one CTA (byte offsets) for n discs, nd of them its own.
+struct ClusterSmem {
+  size_t pos, vel, posf, shear, ref, rest, kcoef, pinv, npos, nvel, acc, warp, other, bond, alive, part, flags, total;
+};
+
+__host__ __device__ inline ClusterSmem cluster_smem(int n, int nd, int warps, int copies, bool kc) {
+  ClusterSmem L;
+  size_t o = 0;
+  const size_t N = (size_t)n, D = (size_t)nd;
+  auto take = [&](size_t bytes) {
+    const size_t at = o;
+    o += (bytes + 15) & ~size_t(15);
+    return at;
+  };
+  L.pos = take(copies * N * 16);
+  L.vel = take(copies * N * 16);
+  L.posf = take(copies * N * 8);
+  L.shear = take(N * 8);
+  L.ref = take(D * kGroup * 16);
+  L.rest = take(D * kGroup * 8);
+  L.kcoef = take(kc ? D * kGroup * 8 : 0);
+  L.pinv = take(D * 32);
+  L.npos = take(copies == 1 ? D * 16 : 0);
+  L.nvel = take(copies == 1 ? D * 16 : 0);
+  L.acc = take(D * kAcc * 8);
+  // per warp: force terms [4][kList] double2 (the shear products [4][4][8] share it),
+  // correction terms [4][8] double2, near pairs [4][kList] int2
+  L.warp = take((size_t)warps * 4 * (kList * 16 + kGroup * 16 + kList * 8));
+  L.other = take(D * kGroup * 4);
+  L.bond = take(D * kGroup * 4);
+  L.alive = take(D * kGroup);
+  L.part = take((size_t)kMaxCluster * kAcc * 8);
+  L.flags = take((size_t)kMaxCluster * 16);
+  L.total = o;
+  return L;
+}
+
+// Force terms of disc k by one lane in scan order (more terms than the lists
+// hold): the loop of icedem_kernel.
+struct SerialSum {
+  double fx, fy, diss;
+};
+
+__device__ __noinline__ SerialSum pair_terms_serial(const Params& P, const Topo& T, int n, int k, const double2* spos,
+                                                    const double2* svel, const float2* sposf, const double2* gpos0,
+                                                    const unsigned char* alive_slots, double fx, double fy,
+                                                    float pre2) {
+  const double eps = 2.220446049250313e-16, two_r = 2.0 * P.radius;
+  const float2 pkf = sposf[k];
+  double diss = 0.0;
+  int cur = T.inc_off[k];
+  const int cur_end = T.inc_off[k + 1];
+  for (int t = 1; t < n; ++t) {
+    int j = k + t;
+    if (j >= n) j -= n;
+    bool alive = false;
+    if (cur < cur_end && T.inc_other[cur] == j) {
+      alive = alive_slots[cur - T.inc_off[k]] != 0;
+      ++cur;
+    }
+    if (!alive) {
+      const float ddx = sposf[j].x - pkf.x, ddy = sposf[j].y - pkf.y;
+      if (ddx * ddx + ddy * ddy > pre2) continue;
+    }
+    const int lo = k < j ? k : j, hi = k < j ? j : k;
+    const double dx = spos[hi].x - spos[lo].x, dy = spos[hi].y - spos[lo].y;
+    const double d = sqrt(fma(dy, dy, dx * dx));
+    double nx, ny;
+    if (d > 0.0) {
+      const double dcl = fmax(d, eps);
+      nx = dx / dcl;
+      ny = dy / dcl;
+    } else {
+      const double ix = gpos0[hi].x - gpos0[lo].x, iy = gpos0[hi].y - gpos0[lo].y;
+      const double id = sqrt(fma(iy, iy, ix * ix));
+      nx = ix / id;
+      ny = iy / id;
+    }
+    double mag;
+    if (alive) {
+      mag = P.kb * (d - T.rest[T.inc_bond[cur - 1]]);
+    } else {
+      const double ov = fmax(two_r - d, 0.0);
+      if (!(ov > 0.0)) continue;
+      const double vn = (svel[hi].x - svel[lo].x) * nx + (svel[hi].y - svel[lo].y) * ny;
+      const double rep = fmax(P.kc * ov - P.cdamp * vn, 0.0);
+      mag = -rep;
+      if (k == lo) diss += (rep - P.kc * ov) * (-vn);
+    }
+    const double pfx = mag * nx, pfy = mag * ny;
+    fx += k == lo ? pfx : -pfx;
+    fy += k == lo ? pfy : -pfy;
+  }
+  return SerialSum{fx, fy, diss};
+}
+
+// Unit vector from lo to hi, and their distance.
+__device__ __forceinline__ double pair_normal(const double2* spos, const double2* gpos0, int lo, int hi, double& nx,
+                                              double& ny) {
+  const double eps = 2.220446049250313e-16;
+  const double dx = spos[hi].x - spos[lo].x, dy = spos[hi].y - spos[lo].y;
+  const double d = sqrt(fma(dy, dy, dx * dx));
+  if (d > 0.0) {
+    const double dcl = fmax(d, eps);
+    nx = dx / dcl;
+    ny = dy / dcl;
+  } else {
+    const double ix = gpos0[hi].x - gpos0[lo].x, iy = gpos0[hi].y - gpos0[lo].y;
+    const double id = sqrt(fma(iy, iy, ix * ix));
+    nx = ix / id;
+    ny = iy / id;
+  }
+  return d;
+}
+
+__global__ void __launch_bounds__((kClusterWarps + 1) * 32, 1)
+    icedem_cluster_kernel(Params P, Topo T, tdem_icedem_state S, const double2* __restrict__ loads, int mode,
+                          int n_steps, double time, double2* __restrict__ out_force, double* __restrict__ out_reaction,
+                          double* __restrict__ ledger, Mailbox* __restrict__ mbox, int per_cta, int copies) {
+  namespace cg = cooperative_groups;
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double s_max[kClusterWarps * 2];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), nc = (int)cluster.num_blocks();
+  const int n = P.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int warps = (int)(blockDim.x >> 5) - 1;  // the last warp keeps the ledger
+  const int k0 = min(n, rank * per_cta), nd = min(n, k0 + per_cta) - k0;
+  const ClusterSmem Y = cluster_smem(n, per_cta, warps, copies, T.kcoef != nullptr);
+  double2* const spos = reinterpret_cast<double2*>(smem + Y.pos);  // [copies][n]
+  double2* const svel = reinterpret_cast<double2*>(smem + Y.vel);
+  float2* const sposf = reinterpret_cast<float2*>(smem + Y.posf);
+  double* const sshear = reinterpret_cast<double*>(smem + Y.shear);
+  double2* const sref = reinterpret_cast<double2*>(smem + Y.ref);
+  double* const srest = reinterpret_cast<double*>(smem + Y.rest);
+  double* const skc = reinterpret_cast<double*>(smem + Y.kcoef);
+  Mat2* const spinv = reinterpret_cast<Mat2*>(smem + Y.pinv);
+  double2* const npos = reinterpret_cast<double2*>(smem + Y.npos);
+  double2* const nvel = reinterpret_cast<double2*>(smem + Y.nvel);
+  double* const sacc = reinterpret_cast<double*>(smem + Y.acc);
+  int* const sother = reinterpret_cast<int*>(smem + Y.other);  // partner of each bond slot, -1: none
+  int* const sbond = reinterpret_cast<int*>(smem + Y.bond);
+  unsigned char* const salive = smem + Y.alive;
+  double* const spart = reinterpret_cast<double*>(smem + Y.part);  // CTA 0: [nc][kAcc]
+  int* const sflag = reinterpret_cast<int*>(smem + Y.flags);       // [2][nc]: non-finite, by step parity
+  unsigned char* const wsm = smem + Y.warp + (size_t)min(warp, warps - 1) * 4 * (kList * 16 + kGroup * 16 + kList * 8);
+  const int g = lane >> 3, l = lane & 7;
+  double2* const flist = reinterpret_cast<double2*>(wsm) + g * kList;
+  double* const sprod = reinterpret_cast<double*>(wsm) + g * 4 * kGroup;
+  double2* const fcorr = reinterpret_cast<double2*>(wsm + 4 * kList * 16) + g * kGroup;
+  int2* const near = reinterpret_cast<int2*>(wsm + 4 * (kList * 16 + kGroup * 16)) + g * kList;
+
+  double2* gpos = reinterpret_cast<double2*>(S.positions);
+  double2* gvel = reinterpret_cast<double2*>(S.velocities);
+  const double2* gpos0 = reinterpret_cast<const double2*>(S.initial_positions);
+
+  for (int k = tid; k < n; k += blockDim.x) {
+    const double2 p = gpos[k];
+    spos[k] = p;
+    svel[k] = gvel[k];
+    sposf[k] = make_float2((float)p.x, (float)p.y);
+  }
+  for (int q = tid; q < nd * kGroup; q += blockDim.x) {
+    const int k = k0 + q / kGroup, e = T.inc_off[k] + (q & 7);
+    const bool has = e < T.inc_off[k + 1];
+    const int b = has ? T.inc_bond[e] : 0;
+    sother[q] = has ? T.inc_other[e] : -1;
+    sbond[q] = b;
+    salive[q] = has && S.alive[T.bpair[b]] ? 1 : 0;
+    if (has) {
+      sref[q] = T.ref[b];
+      srest[q] = T.rest[b];
+      if (T.kcoef) skc[q] = T.kcoef[b];
+    }
+  }
+  for (int q = tid; q < nd; q += blockDim.x) spinv[q] = T.pinv[k0 + q];
+  for (int q = tid; q < 2 * kMaxCluster; q += blockDim.x) sflag[q] = 0;
+  __syncthreads();
+
+  const double two_r = 2.0 * P.radius;
+  const float pre2 = (float)(two_r * two_r) * 1.001f + 1e-30f;
+  // a disc this far from the circular tool carries no tool force (FP32 guard band as above)
+  const double reach = P.radius + P.tool_radius;
+  const float tool2 = (float)(reach * reach) * 1.001f + 1e-30f;
+  double max_t = -1e300, max_s = -1e300;  // largest strains of surviving bonds (lo side)
+  const bool keeper = warp == warps;       // ledger warp
+  // CTA 0's ledger warp: running totals (lane q < 8: impulse component q)
+  double imp = 0.0, release = 0.0, acquired = 0.0, twork = 0.0, damp = 0.0, ework = 0.0;
+  double tot = 0.0, power_d = 0.0, power_t = 0.0, last_work = 0.0, last_t0 = 0.0;
+  constexpr int kImpulse[8] = {TDEM_L_TOOL_IMPULSE_X,    TDEM_L_TOOL_IMPULSE_Y, TDEM_L_SUPPORT_IMPULSE_X,
+                               TDEM_L_SUPPORT_IMPULSE_Y, TDEM_L_DRAG_IMPULSE_X, TDEM_L_DRAG_IMPULSE_Y,
+                               TDEM_L_EXTERNAL_IMPULSE_X, TDEM_L_EXTERNAL_IMPULSE_Y};
+  const bool books = keeper && rank == 0;
+  if (books) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (lane == q) imp = ledger[kImpulse[q]];
+    release = ledger[TDEM_L_FRACTURE_RELEASE];
+    acquired = ledger[TDEM_L_CONTACT_ACQUIRED];
+    twork = ledger[TDEM_L_TOOL_WORK];
+    damp = ledger[TDEM_L_DAMPING_DISSIPATION];
+    ework = ledger[TDEM_L_EXTERNAL_WORK];
+  }
+  // this CTA's sums of the last force phase, one lane per term, to CTA 0
+  auto send_sums = [&]() {
+    if (!keeper || lane >= kAcc) return;
+    double s = 0.0;
+    for (int q = 0; q < nd; ++q) s += sacc[q * kAcc + lane];
+    cluster.map_shared_rank(spart, 0)[rank * kAcc + lane] = s;
+  };
+  // CTA 0: the ledger of the step that began at t0 (full: with the Euler part)
+  auto book = [&](double t0, bool full) {
+    if (!books) return;
+    double s = 0.0;
+    if (lane < kAcc)
+      for (int r = 0; r < nc; ++r) s += spart[r * kAcc + lane];
+    tot = s;
+    auto of = [&](int c) { return __shfl_sync(kAll, s, c); };
+    const double rx = -of(0), ry = -of(1);
+    const double tvx = P.hull_m ? P.hull_vel_x : P.tool_vel_x, tvy = P.hull_m ? P.hull_vel_y : P.tool_vel_y;
+    power_d = (of(8) + (-of(9))) + P.drag * of(10);
+    power_t = -(rx * tvx + ry * tvy);
+    release += of(12);
+    acquired += of(13);
+    if (T.kcoef) release += of(14);
+    if (full) {
+      const double coef = lane < 2 ? 1.0 : lane < 4 ? -1.0 : lane < 6 ? -P.drag : 1.0;
+      imp = imp + P.dt * (coef * s);
+      last_work = loads ? of(15) : 0.0;
+      ework += last_work;
+      twork += P.dt * power_t;
+      damp += P.dt * power_d;
+      last_t0 = t0;
+    }
+  };
+
+  int steps_done = 0, buf = 0;
+  bool bad = false;
+  const int total = mode == 1 ? 1 : n_steps;
+  cluster.sync();  // every CTA's shared memory is set up
+  for (int step = 0; step < total; ++step) {
+    const double2* pos = spos + (size_t)buf * n;
+    const double2* vel = svel + (size_t)buf * n;
+    const float2* posf = sposf + (size_t)buf * n;
+    // ---- objective local shear strain (dem.py:182-208)
+    if (keeper) {
+      if (step > 0) send_sums();
+    } else {
+      for (int q0 = warp * 4; q0 < nd; q0 += warps * 4) {
+        const int q = q0 + g;
+        const bool on = q < nd;
+        const int k = k0 + q;
+        const int o = on ? sother[q * kGroup + l] : -1;
+        if (o >= 0) {
+          const int lo = min(k, o), hi = max(k, o);
+          const double2 r = sref[q * kGroup + l];
+          const double cx = pos[hi].x - pos[lo].x, cy = pos[hi].y - pos[lo].y;
+          sprod[l] = cx * r.x;
+          sprod[kGroup + l] = cx * r.y;
+          sprod[2 * kGroup + l] = cy * r.x;
+          sprod[3 * kGroup + l] = cy * r.y;
+        }
+        const int deg = __popc(__ballot_sync(kAll, o >= 0) >> (8 * g) & 0xFFu);
+        __syncwarp();
+        const int c = l & 3;
+        double sum = 0.0;
+#pragma unroll
+        for (int e = 0; e < kGroup; ++e)
+          if (e < deg) sum += sprod[c * kGroup + e];
+        auto of = [&](double x, int src) { return __shfl_sync(kAll, x, src, kGroup); };
+        // lane c = 2 a + b: f_ab = c_a0 pinv_0b + c_a1 pinv_1b
+        const Mat2 m = spinv[on ? q : 0];
+        const double ca0 = of(sum, c & 2), ca1 = of(sum, (c & 2) + 1);
+        const double f = ca0 * ((c & 1) ? m.y : m.x) + ca1 * ((c & 1) ? m.w : m.z);
+        const double f00 = of(f, 0), f01 = of(f, 1), f10 = of(f, 2), f11 = of(f, 3);
+        // lane 0: e00, lane 1: e01, lane 2: e11
+        const double u0 = c == 2 ? f01 : f00, u1 = c == 0 ? f00 : f01;
+        const double w0 = c == 2 ? f11 : f10, w1 = c == 0 ? f10 : f11;
+        const double uw = u0 * u1 + w0 * w1;
+        const double ee = 0.5 * (c == 1 ? uw : uw - 1.0);
+        const double e00 = of(ee, 0), e01 = of(ee, 1), e11 = of(ee, 2);
+        const double dd = e00 - e11;
+        const double sh = sqrt(dd * dd + 4.0 * (e01 * e01));
+        if (on)
+          for (int r = l; r < nc; r += kGroup) cluster.map_shared_rank(sshear, r)[k] = sh;
+        __syncwarp();
+      }
+    }
+    cluster.sync();
+    // ---- break test, forces, and the Euler step (dem.py:243-382)
+    if (keeper) {
+      if (step > 0) book(time - P.dt, true);
+    } else {
+      for (int q0 = warp * 4; q0 < nd; q0 += warps * 4) {
+        const int q = q0 + g;
+        const bool on = q < nd;
+        const int k = k0 + q, slot = q * kGroup + l;
+        const int o = on ? sother[slot] : -1;
+        const int lo = min(k, o), hi = max(k, o);
+        bool alive = o >= 0 && salive[slot];
+        double nx = 0.0, ny = 0.0, ext = 0.0, brk0 = 0.0, brk1 = 0.0, brk2 = 0.0;
+        bool breaks = false;
+        if (alive) {
+          const double d = pair_normal(pos, gpos0, lo, hi, nx, ny);
+          ext = d - srest[slot];
+          const double ts = ext / srest[slot];
+          const double bs = 0.5 * (sshear[lo] + sshear[hi]);
+          const bool tf = ts > P.eps_t, sf = bs > P.eps_s;
+          breaks = tf || sf;
+          if (breaks) {
+            alive = false;
+            salive[slot] = 0;
+            if (k == lo) {
+              const long long p = T.bpair[sbond[slot]];
+              const double energy = (0.5 * P.kb) * (ext * ext);
+              S.alive[p] = 0;
+              S.failure_mode[p] = (uint8_t)((tf ? 1 : 0) + 2 * (sf ? 1 : 0));
+              S.failure_time_s[p] = time;
+              S.failure_extension_m[p] = ext;
+              brk0 = energy;
+              double e = energy;
+              if (T.kcoef) {
+                brk2 = (0.5 * (skc[slot] - P.kb)) * (ext * ext);
+                e = energy + brk2;
+              }
+              S.failure_energy_J[p] = e;
+              const double ov = fmax(two_r - d, 0.0);
+              brk1 = (0.5 * P.kc) * (ov * ov);
+            }
+          } else if (k == lo) {
+            max_t = fmax(max_t, ts);
+            max_s = fmax(max_s, bs);
+          }
+        }
+        // places of the force terms in scan order: partner j = k + 1 + 8 c + lane (mod n)
+        const int key = o >= 0 ? (o > k ? o - k - 1 : o - k - 1 + n) : -1;
+        const float2 pk = on ? posf[k] : make_float2(0.0f, 0.0f);
+        int count = 0, nnear = 0, place = -1;
+        for (int c = 0; c * kGroup < n - 1; ++c) {
+          const int t = c * kGroup + l;
+          int j = k + 1 + t;
+          if (j >= n) j -= n;
+          const unsigned bonds =
+              __reduce_or_sync(kAll, alive && (key >> 3) == c ? 1u << (8 * g + (key & 7)) : 0u) >> (8 * g) & 0xFFu;
+          bool close = false;
+          if (on && t < n - 1) {
+            const float dx = posf[j].x - pk.x, dy = posf[j].y - pk.y;
+            close = !(dx * dx + dy * dy > pre2) && !((bonds >> l) & 1u);
+          }
+          const unsigned nears = __ballot_sync(kAll, close) >> (8 * g) & 0xFFu;
+          const unsigned terms = bonds | nears;
+          if (alive && (key >> 3) == c) place = count + __popc(terms & ((1u << (key & 7)) - 1u));
+          if (close) {
+            const int at = nnear + __popc(nears & ((1u << l) - 1u));
+            if (at < kList) near[at] = make_int2(j, count + __popc(terms & ((1u << l) - 1u)));
+          }
+          count += __popc(terms);
+          nnear += __popc(nears);
+        }
+        const bool full = count > kList;  // more terms than the lists hold: summed by one lane below
+        __syncwarp();
+        if (alive && !full) {
+          const double mag = P.kb * ext;
+          const double px = mag * nx, py = mag * ny;
+          flist[place] = k == lo ? make_double2(px, py) : make_double2(-px, -py);
+        }
+        double diss = 0.0;
+        const int rounds = __reduce_max_sync(kAll, full ? 0 : nnear);
+        for (int b = 0; b < rounds; b += kGroup) {
+          double pd = 0.0;
+          if (!full && b + l < nnear) {
+            const int j = near[b + l].x, at = near[b + l].y;
+            const int a = min(k, j), z = max(k, j);
+            double ux, uy;
+            const double d = pair_normal(pos, gpos0, a, z, ux, uy);
+            const double ov = fmax(two_r - d, 0.0);
+            double px = 0.0, py = 0.0;
+            if (ov > 0.0) {
+              const double vn = (vel[z].x - vel[a].x) * ux + (vel[z].y - vel[a].y) * uy;
+              const double rep = fmax(P.kc * ov - P.cdamp * vn, 0.0);
+              px = -rep * ux;
+              py = -rep * uy;
+              if (k == a)
+                pd = (rep - P.kc * ov) * (-vn);
+              else {
+                px = -px;
+                py = -py;
+              }
+            }
+            flist[at] = make_double2(px, py);
+          }
+          if (__any_sync(kAll, pd != 0.0))
+            for (int e = 0; e < kGroup; ++e) diss += __shfl_sync(kAll, pd, e, kGroup);
+        }
+        if (T.kcoef) {
+          // per-bond stiffness (calibrated_dem.py:70-79): (k_b - k) * extension * n
+          // of each surviving bond, after the other forces
+          const double m = alive ? (skc[slot] - P.kb) * ext : 0.0;
+          fcorr[l] = k == lo ? make_double2(m * nx, m * ny) : make_double2(-(m * nx), -(m * ny));
+        }
+        const unsigned live = __ballot_sync(kAll, alive) >> (8 * g) & 0xFFu;
+        __syncwarp();
+        // lane 0 of the group: x, lane 1: y (the others repeat them)
+        const bool y = l & 1;
+        const double2 p0 = on ? pos[k] : make_double2(0.0, 0.0), v0 = on ? vel[k] : make_double2(0.0, 0.0);
+        double f = (-P.drag) * (y ? v0.y : v0.x);
+        if (full) {
+          SerialSum s{0.0, 0.0, 0.0};
+          if (on && l == 0)
+            s = pair_terms_serial(P, T, n, k, pos, vel, posf, gpos0, salive + q * kGroup, (-P.drag) * v0.x,
+                                  (-P.drag) * v0.y, pre2);
+          const unsigned mine = 0xFFu << (8 * g);
+          const double sx = __shfl_sync(mine, s.fx, 0, kGroup), sy = __shfl_sync(mine, s.fy, 0, kGroup);
+          diss = __shfl_sync(mine, s.diss, 0, kGroup);
+          f = y ? sy : sx;
+        } else {
+          for (int e = 0; e < count; ++e) f += y ? flist[e].y : flist[e].x;
+        }
+        __syncwarp();
+        // tool
+        double tdiss = 0.0;
+        double2 tf = make_double2(0.0, 0.0);
+        bool tooled = on && l == 0;
+        if (tooled && P.hull_m == 0) {
+          const float dx = pk.x - (float)(P.tool_start_x + time * P.tool_vel_x);
+          const float dy = pk.y - (float)(P.tool_start_y + time * P.tool_vel_y);
+          tooled = !(dx * dx + dy * dy > tool2 + 1e-5f * (pk.x * pk.x + pk.y * pk.y + dx * dx + dy * dy));
+        }
+        if (tooled) tf = tool_contact(P, T, p0, v0, time, tdiss);
+        if (__any_sync(kAll, tooled)) {
+          tf.x = __shfl_sync(kAll, tf.x, 0, kGroup);
+          tf.y = __shfl_sync(kAll, tf.y, 0, kGroup);
+          f += y ? tf.y : tf.x;
+        }
+        double2 ld = make_double2(0.0, 0.0);
+        if (loads) {
+          if (on) ld = loads[k];
+          f += y ? ld.y : ld.x;
+        }
+        if (T.kcoef) {
+          for (int e = 0; e < kGroup; ++e)
+            if ((live >> e) & 1u) f += y ? fcorr[e].y : fcorr[e].x;
+        }
+        // semi-implicit Euler
+        const bool fixed = on && S.fixed[k] != 0;
+        const double vc = y ? v0.y : v0.x, pc = y ? p0.y : p0.x;
+        double v1 = vc + (P.dt * f) / P.mass;
+        if (fixed) v1 = 0.0;
+        double p1 = pc + P.dt * v1;
+        if (fixed) p1 = y ? gpos0[k].y : gpos0[k].x;
+        const double fx = __shfl_sync(kAll, f, 0, kGroup), fy = __shfl_sync(kAll, f, 1, kGroup);
+        const double vx = __shfl_sync(kAll, v1, 0, kGroup), vy = __shfl_sync(kAll, v1, 1, kGroup);
+        const double px = __shfl_sync(kAll, p1, 0, kGroup), py = __shfl_sync(kAll, p1, 1, kGroup);
+        // ledger terms
+        if (__any_sync(kAll, breaks)) {
+          double a = 0.0, b = 0.0, c = 0.0;
+          for (int e = 0; e < kGroup; ++e) {
+            a += __shfl_sync(kAll, brk0, e, kGroup);
+            b += __shfl_sync(kAll, brk1, e, kGroup);
+            c += __shfl_sync(kAll, brk2, e, kGroup);
+          }
+          brk0 = a;
+          brk1 = b;
+          brk2 = c;
+        }
+        if (on) {
+          double* acc = sacc + q * kAcc;
+          if (l == 0) {
+            acc[0] = tf.x;
+            acc[8] = diss;
+          } else if (l == 1) {
+            acc[1] = tf.y;
+            acc[12] = brk0;
+            acc[13] = brk1;
+            acc[14] = brk2;
+          } else if (l == 2) {
+            acc[2] = fixed ? fx : 0.0;
+            acc[3] = fixed ? fy : 0.0;
+          } else if (l == 3) {
+            acc[4] = v0.x;
+            acc[5] = v0.y;
+            acc[10] = v0.x * v0.x + v0.y * v0.y;
+          } else if (l == 4) {
+            acc[6] = ld.x;
+            acc[7] = ld.y;
+          } else if (l == 5) {
+            acc[11] = loads ? p0.x * ld.y - p0.y * ld.x : 0.0;
+            acc[15] = loads ? ld.x * (px - p0.x) + ld.y * (py - p0.y) : 0.0;
+          }
+          if (l == 0) acc[9] = tdiss;
+          if (mode == 1) {
+            if (l == 0) out_force[k] = make_double2(fx, fy);
+          } else {
+            if (!(isfinite(px) && isfinite(py) && isfinite(vx) && isfinite(vy)))
+              for (int r = l; r < nc; r += kGroup) cluster.map_shared_rank(sflag, r)[(step & 1) * kMaxCluster + rank] = 1;
+            if (copies == 2) {
+              const size_t at = (size_t)(buf ^ 1) * n + k;
+              for (int r = l; r < nc; r += kGroup) {
+                cluster.map_shared_rank(spos, r)[at] = make_double2(px, py);
+                cluster.map_shared_rank(svel, r)[at] = make_double2(vx, vy);
+                cluster.map_shared_rank(sposf, r)[at] = make_float2((float)px, (float)py);
+              }
+            } else if (l == 0) {
+              npos[q] = make_double2(px, py);
+              nvel[q] = make_double2(vx, vy);
+            }
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (mode == 1) break;
+    if (copies == 1) {
+      cluster.sync();  // every CTA is done with the old positions
+      for (int q = tid; q < nd * nc; q += blockDim.x) {
+        const int d = q / nc, r = q - d * nc, k = k0 + d;
+        const double2 p = npos[d];
+        cluster.map_shared_rank(spos, r)[k] = p;
+        cluster.map_shared_rank(svel, r)[k] = nvel[d];
+        cluster.map_shared_rank(sposf, r)[k] = make_float2((float)p.x, (float)p.y);
+      }
+    }
+    cluster.sync();
+    if (copies == 2) buf ^= 1;
+    time = time + P.dt;
+    steps_done = step + 1;
+    const int* fl = sflag + (step & 1) * kMaxCluster;
+    for (int r = 0; r < nc; ++r) bad = bad || fl[r] != 0;
+    if (bad) break;
+  }
+  // the last step's ledger, the largest strains, the state
+  if (mode == 1) cluster.sync();
+  send_sums();
+  if (!keeper) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      max_t = fmax(max_t, __shfl_down_sync(kAll, max_t, off));
+      max_s = fmax(max_s, __shfl_down_sync(kAll, max_s, off));
+    }
+    if (lane == 0) {
+      s_max[2 * warp] = max_t;
+      s_max[2 * warp + 1] = max_s;
+    }
+  }
+  if (mode == 0)
+    for (int q = tid; q < nd; q += blockDim.x) {
+      gpos[k0 + q] = spos[(size_t)buf * n + k0 + q];
+      gvel[k0 + q] = svel[(size_t)buf * n + k0 + q];
+    }
+  __syncthreads();
+  double* const peak = reinterpret_cast<double*>(sflag);  // CTA 0: [nc][2] (16 bytes each)
+  cluster.sync();  // the flags are no longer read: reuse their words
+  if (tid == 0) {
+    double a = -1e300, b = -1e300;
+    for (int w = 0; w < warps; ++w) {
+      a = fmax(a, s_max[2 * w]);
+      b = fmax(b, s_max[2 * w + 1]);
+    }
+    double* to = cluster.map_shared_rank(peak, 0) + 2 * rank;
+    to[0] = a;
+    to[1] = b;
+  }
+  cluster.sync();
+  if (!books) return;
+  book(time - P.dt, mode == 0);
+  double a = -1e300, b = -1e300;
+  for (int r = 0; r < nc; ++r) {
+    a = fmax(a, peak[2 * r]);
+    b = fmax(b, peak[2 * r + 1]);
+  }
+  auto of = [&](int c) { return __shfl_sync(kAll, tot, c); };
+  const double t0 = of(0), t1 = of(1), t2 = of(2), t3 = of(3), t6 = of(6), t7 = of(7), t11 = of(11);
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (lane == q && mode == 0) ledger[kImpulse[q]] = imp;
+  if (lane != 0) return;
+  // the smallest margin of a surviving bond belongs to the largest strain (the
+  // margin falls with the strain, its rounding included)
+  double margin = 1e300;
+  if (a > -1e300) margin = fmin((P.eps_t - a) / P.eps_t, (P.eps_s - b) / P.eps_s);
+  ledger[TDEM_L_MIN_BREAK_MARGIN] = fmin(ledger[TDEM_L_MIN_BREAK_MARGIN], margin);
+  ledger[TDEM_L_FRACTURE_RELEASE] = release;
+  ledger[TDEM_L_CONTACT_ACQUIRED] = acquired;
+  ledger[TDEM_L_DAMPING_POWER] = power_d;
+  ledger[TDEM_L_TOOL_POWER] = power_t;
+  if (mode == 1) {
+    out_reaction[0] = -t0;
+    out_reaction[1] = -t1;
+  } else {
+    ledger[TDEM_L_EXTERNAL_WORK] = ework;
+    ledger[TDEM_L_TOOL_WORK] = twork;
+    ledger[TDEM_L_DAMPING_DISSIPATION] = damp;
+    ledger[TDEM_L_LAST_SUPPORT_X] = -t2;
+    ledger[TDEM_L_LAST_SUPPORT_Y] = -t3;
+    ledger[TDEM_L_LAST_REACTION_X] = -t0;
+    ledger[TDEM_L_LAST_REACTION_Y] = -t1;
+    ledger[TDEM_L_LAST_EXTERNAL_X] = t6;
+    ledger[TDEM_L_LAST_EXTERNAL_Y] = t7;
+    ledger[TDEM_L_LAST_EXTERNAL_WORK] = last_work;
+    ledger[TDEM_L_LAST_EXTERNAL_MOMENT] = loads ? t11 : 0.0;
+    ledger[TDEM_L_LAST_TIME_START] = last_t0;
+    ledger[TDEM_L_LAST_TIME_END] = last_t0 + P.dt;
+  }
+  mbox->steps_done = steps_done;
+  mbox->status = bad ? TDEM_ERR_NONFINITE : TDEM_OK;
+}
+
+// ---------------------------------------------------------------------------
+// The same step on one CTA, one thread per disc, for discs of more than
+// kGroup bonds. mode 0: n_steps full steps; mode 1: one force
 // evaluation (dem.py:226-345) written to out_force / out_reaction.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(512) icedem_kernel(Params P, Topo T, tdem_icedem_state S,
@@ -636,6 +1273,8 @@ struct tdem_icedem {
   double* ledger_host = nullptr;
   int threads = 32;
   size_t smem = 0;
+  // cluster form: CTAs, discs of each, threads of each, copies of the positions
+  int cluster = 0, per_cta = 0, cthreads = 0, copies = 0;
   std::string err;
 };
 
@@ -692,6 +1331,69 @@ int upload(std::string* err, T** dst, const std::vector<T>& src) {
   TDEM_CUDA_TRY(err, cudaMalloc(reinterpret_cast<void**>(dst), bytes));
   if (!src.empty()) TDEM_CUDA_TRY(err, cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
   return TDEM_OK;
+}
+
+cudaLaunchConfig_t cluster_config(const tdem_icedem* h, cudaLaunchAttribute* at, size_t smem, cudaStream_t s) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)h->cluster);
+  c.blockDim = dim3((unsigned)h->cthreads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)h->cluster;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return c;
+}
+
+size_t cluster_bytes(const tdem_icedem* h, bool kcoef) {
+  return tdem::icedem::cluster_smem(h->n, h->per_cta, h->cthreads / 32 - 1, h->copies, kcoef).total;
+}
+
+// Shape of the cluster form: as many CTAs as the discs fill with one warp each
+// (four discs a warp), at most 16; both copies of the positions while they fit
+// (a step then needs two cluster barriers, else three). h->cluster stays 0
+// where no such cluster can run: the one-CTA kernel steps then.
+void plan_cluster(tdem_icedem* h, bool kcoef) {
+  using namespace tdem::icedem;
+  h->cluster = 0;
+  int dev = 0, smem_max = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncSetAttribute(icedem_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(icedem_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 1024) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  for (int want : {kMaxCluster, 8}) {
+    int nc = 1;
+    while (nc < want && nc * 4 < h->n) nc *= 2;
+    const int per = (h->n + nc - 1) / nc;
+    for (int copies : {2, 1}) {
+      tdem_icedem shape = {};
+      shape.n = h->n;
+      shape.cluster = nc;
+      shape.per_cta = per;
+      shape.cthreads = (std::min(kClusterWarps, (per + 3) / 4) + 1) * 32;
+      shape.copies = copies;
+      const size_t smem = cluster_bytes(&shape, kcoef);
+      if (smem > (size_t)smem_max - 1024) continue;
+      cudaLaunchAttribute at;
+      const cudaLaunchConfig_t c = cluster_config(&shape, &at, smem, nullptr);
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, icedem_cluster_kernel, &c) != cudaSuccess || fit < 1) {
+        cudaGetLastError();
+        continue;
+      }
+      h->cluster = nc;
+      h->per_cta = per;
+      h->cthreads = shape.cthreads;
+      h->copies = copies;
+      return;
+    }
+  }
 }
 
 }  // namespace
@@ -854,6 +1556,9 @@ int tdem_icedem_create(const tdem_icedem_config* cfg, const double* x0, tdem_ice
     tdem_icedem_destroy(h);
     return tdem::fail(err, TDEM_ERR_CUDA, std::string("smem attribute: ") + cudaGetErrorString(e));
   }
+  int degree = 0;
+  for (int k = 0; k < n; ++k) degree = std::max(degree, inc_off[k + 1] - inc_off[k]);
+  if (degree <= kGroup) plan_cluster(h, false);
   *out = h;
   return TDEM_OK;
 }
@@ -873,7 +1578,9 @@ int tdem_icedem_set_bond_stiffness(tdem_icedem* h, const double* k_host, int cou
     cudaFree(h->kcoef);
     h->kcoef = nullptr;
   }
-  return upload(&h->err, &h->kcoef, k);
+  const int rc = upload(&h->err, &h->kcoef, k);
+  if (rc == TDEM_OK && h->cluster > 0) plan_cluster(h, true);  // the coefficients take shared memory too
+  return rc;
 }
 
 int tdem_icedem_bond_pairs(const tdem_icedem* h, int64_t* out) {
@@ -892,6 +1599,15 @@ static int launch(tdem_icedem* h, const tdem_icedem_state* st, const double* loa
   Topo T{h->bi, h->bj, h->bpair, h->rest, h->ref, h->inc_off, h->inc_bond, h->inc_other, h->pinv, h->hull,
          h->kcoef};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (h->cluster > 0) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t c = cluster_config(h, &at, cluster_bytes(h, h->kcoef != nullptr), s);
+    TDEM_CUDA_TRY(&h->err, cudaLaunchKernelEx(&c, icedem_cluster_kernel, h->P, T, *st,
+                                              reinterpret_cast<const double2*>(loads), mode, n_steps, time,
+                                              reinterpret_cast<double2*>(out_force), out_reaction, h->ledger, h->mbox,
+                                              h->per_cta, h->copies));
+    return TDEM_OK;
+  }
   icedem_kernel<<<1, h->threads, h->smem, s>>>(h->P, T, *st, reinterpret_cast<const double2*>(loads),
                                                mode, n_steps, time,
                                                reinterpret_cast<double2*>(out_force), out_reaction,
