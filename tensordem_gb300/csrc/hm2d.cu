@@ -324,6 +324,7 @@ struct Engine final : EngineBase {
     RunFn<T> fn = nullptr;
     int pb = 0, grid = 0, threads = 0;  // discs per block (one per thread), blocks, threads
     size_t smem = 0;
+    int pairs = 0;  // pairs a block without bonds has room for
   };
   RunPlan run0, runp;
   bool primed = false;
@@ -486,20 +487,35 @@ struct Engine final : EngineBase {
     auto warps = [](long long n) { return (int)((n + 31) / 32) * 32; };
     for (int build = 0; build < 3; ++build) {
       const bool local = build == 0, big = build == 2;
-      int most = run_block<T>(f, big) - extra;
+      const int threads = run_block<T>(f, big);
+      int most = threads - extra;
       if (local) most = std::min(most, f ? kRunLocalBonds : kRunLocal);
       const int pb = local ? warps(P.n) : std::max(std::min(kRunDiscs, most), warps((P.n + sms - 1) / sms));
       if (pb > most) continue;
-      const size_t smem = run_layout<T>(P.W, f ? P.BMAX : 0, pb, local ? 1 : 0, P.n).total;
+      // without bonds: the pairs that fit beside the discs, and a thread for each
+      // where the block can have them; with bonds a thread per disc
+      int pairs = 0, nt = pb + extra;
+      size_t smem;
+      if (f) {
+        smem = run_layout<T>(P.W, P.BMAX, pb, local ? 1 : 0, P.n).total;
+      } else {
+        const size_t fixed = pair_layout<T>(P.W, pb, 0).total + 256;
+        const size_t each = sizeof(V4<T>) + sizeof(V2<T>) + 8 + 2 + 1;
+        if (fixed > (size_t)smem_max) continue;
+        pairs = (int)std::min<size_t>(std::min<size_t>((size_t)P.W * pb, 0x7FFF), ((size_t)smem_max - fixed) / each);
+        if (pairs < std::min(P.W, kRunPairs) * pb) continue;
+        smem = std::max(pair_layout<T>(P.W, pb, pairs).total, run_layout<T>(P.W, 0, pb, local ? 1 : 0, P.n).total);
+        nt = std::min(threads, std::max(pb, warps((long long)kRunPairs * pb)));
+      }
       if (smem > (size_t)smem_max) continue;
       RunFn<T> fn = run_fn<T>(f, local, big);
       int per_sm = 0;
       TDEM_CUDA_TRY(&err, cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
-      TDEM_CUDA_TRY(&err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn),
-                                                                        pb + extra, smem));
+      TDEM_CUDA_TRY(&err, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn), nt,
+                                                                        smem));
       if (per_sm < 1) continue;
-      run0 = RunPlan{fn, pb, (P.n + pb - 1) / pb, pb + extra, smem};
+      run0 = RunPlan{fn, pb, (P.n + pb - 1) / pb, nt, smem, pairs};
       break;
     }
     if constexpr (sizeof(T) == 4) {
@@ -587,8 +603,8 @@ struct Engine final : EngineBase {
                            cudaGraphConditionalHandle h, cudaGraphConditionalHandle hl, int cond_bits) {
     cudaGraphNode_t knode;
     if (const RunPlan* r = resident()) {
-      int discs = r->pb;
-      void* args[] = {&P, &B, &h, &hl, &cond_bits, &discs};
+      int discs = r->pb, pairs = r->pairs;
+      void* args[] = {&P, &B, &h, &hl, &cond_bits, &discs, &pairs};
       cudaKernelNodeParams kp = {};
       kp.func = reinterpret_cast<void*>(r->fn);
       kp.gridDim = dim3((unsigned)r->grid);

@@ -150,6 +150,7 @@ struct Ctl {
   // counts them across launches), zeroed one barrier ahead
   unsigned epoch;
   unsigned entries[2];     // indenter partials of the even and odd evaluations
+  unsigned long long candidates;  // candidate slots of all lists (the last rebuild's)
   alignas(128) GridWord word[3];
 };
 

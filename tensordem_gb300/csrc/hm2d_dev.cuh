@@ -1704,8 +1704,9 @@ static __global__ void scan_blocks_kernel(const Ctl* ctl, const int* in, int* ou
 }
 
 // One block; any number of block sums, kScanChunk at a time with a carry.
-static __global__ void scan_top_kernel(const Ctl* ctl, int* block_sums, int n_arg) {
+static __global__ void scan_top_kernel(Ctl* ctl, int* block_sums, int n_arg) {
   if (!ctl->rebuild_pending) return;
+  if (threadIdx.x == 0) ctl->candidates = 0ull;  // counted anew by the list build
   const int nblocks = (scan_count(ctl, n_arg) + kScanChunk - 1) / kScanChunk;
   int carry = 0;
   for (int c0 = 0; c0 < nblocks; c0 += kScanChunk) {
@@ -1852,6 +1853,8 @@ __global__ void build_nbr_kernel(Params<T> P, Bufs<T> B) {
   const V4<T>* pos = B.pos[sp1];
   unsigned* tail = B.nbr[lp1];
   const size_t n = (size_t)P.n;
+  int most = 0;        // largest list and candidates of this thread's discs
+  unsigned sum = 0u;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nn; p += gridDim.x * blockDim.x) {
     const int inst = MULTI ? B.inst[lp1][p] : 0;
     const Params<T>& Q = MULTI ? B.iparams[inst] : P;
@@ -1896,7 +1899,14 @@ __global__ void build_nbr_kernel(Params<T> P, Bufs<T> B) {
       cnt = P.W;
     }
     B.head[lp1][p] = make_uint4((unsigned)cnt, first[0], first[1], first[2]);
-    atomicMax(&ctl->max_cnt, cnt);
+    most = max(most, cnt);
+    sum += (unsigned)cnt;
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if ((threadIdx.x & 31) == 0 && sum) {
+    atomicMax(&ctl->max_cnt, most);
+    atomicAdd(&ctl->candidates, (unsigned long long)sum);
   }
 }
 

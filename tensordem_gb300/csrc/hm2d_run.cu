@@ -53,12 +53,342 @@ __device__ __forceinline__ void book_reaction(const Params<T>& P, const Bufs<T>&
   if (m) *reinterpret_cast<volatile unsigned*>(&B.ctl->entries[par]) = 0u;
 }
 
-template <class T, bool FEAT, bool LOCAL, bool BIG>
-__global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
-    force_kernel_run(Params<T> P, Bufs<T> B, cudaGraphConditionalHandle h_rebuild, cudaGraphConditionalHandle h_loop,
-                     int use_cond, int pb) {
+// One evaluation of a disc from the global arrays (a block whose pairs its
+// shared memory does not hold).
+template <class T>
+__device__ __noinline__ void direct_disc(const Params<T>& P, const Bufs<T>& B, int sp, int lp, int i, int primed,
+                                         long long eval, ThreadLedger<T>& L) {
+  const PlainFetch<T> fetch{B.pos[sp], B.vel[sp]};
+  const V4<T> p = fetch.p(i), v = fetch.v(i);
+  const uint4 hd = B.head[lp][i];
+  V4<T> q0{}, q1{}, q2{};
+  load_head_partners<T>(fetch, hd, q0, q1, q2);
+  process_particle_q<T, kBatch, false, PlainFetch<T>>(P, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, primed, eval, L);
+}
+
+// Exclusive prefix of x over the block's threads and the total.
+__device__ __forceinline__ unsigned block_prefix(unsigned x, unsigned* s_warp, unsigned& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5);
+  unsigned incl = x;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += y;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  unsigned before = 0u;
+  total = 0u;
+  for (int w = 0; w < warps; ++w) {
+    if (w < warp) before += s_warp[w];
+    total += s_warp[w];
+  }
+  __syncthreads();
+  return before + incl - x;
+}
+
+constexpr unsigned kPlaceOwner = 0x8000u;  // this disc is the lower one of the pair
+constexpr unsigned kOutside = 0xFFFFu;     // a partner of another block
+
+template <class T, bool LOCAL, bool BIG>
+__device__ __forceinline__ void run_pairs(const Params<T>& P, const Bufs<T>& B, unsigned char* run_smem,
+                                          cudaGraphConditionalHandle h_rebuild, cudaGraphConditionalHandle h_loop,
+                                          int use_cond, int pb, int mc) {
   constexpr int MODE = kBatch;  // the first evaluation of a state primes it
-  extern __shared__ __align__(16) unsigned char run_smem[];
+  __shared__ unsigned s_vmax[3], s_out[4], s_warp[32];
+  __shared__ int s_bad[3], s_touch[3];
+  Ctl* ctl = B.ctl;
+  const int t = threadIdx.x, lane = t & 31, nt = (int)blockDim.x;
+  const int n = P.n;
+  const int i0 = (int)blockIdx.x * pb, mine = min(pb, n - i0);  // this block's discs
+  const int i = i0 + t;
+  const bool own = t < mine;
+  int sp = ctl->sp;
+  const int lp = ctl->lp;
+  long long eval = ctl->evals;
+  const long long target = ctl->target;
+  float disp = ctl->disp;
+  unsigned epoch = ctl->epoch;
+  if (t < 3) {
+    s_vmax[t] = 0u;
+    s_bad[t] = 0;
+    s_touch[t] = 0;
+  }
+  const PairLayout Y = pair_layout<T>(P.W, pb, mc);
+  V4<T>* const spos = reinterpret_cast<V4<T>*>(run_smem + Y.pos);
+  V4<T>* const svel = reinterpret_cast<V4<T>*>(run_smem + Y.vel);
+  V4<T>* const res = reinterpret_cast<V4<T>*>(run_smem + Y.res);   // force on a, torque per lever, loss
+  V2<T>* const hist = reinterpret_cast<V2<T>*>(run_smem + Y.hist);
+  uint2* const desc = reinterpret_cast<uint2*>(run_smem + Y.desc);  // {disc | partner's place << 16, partner}
+  int* const base = reinterpret_cast<int*>(run_smem + Y.base);     // first pair of each disc
+  unsigned short* const place = reinterpret_cast<unsigned short*>(run_smem + Y.place);  // [W][pb]
+  unsigned short* const touch = reinterpret_cast<unsigned short*>(run_smem + Y.touch);  // touching pairs
+  unsigned char* const on = run_smem + Y.on;  // bit 0: touching, bit 1: stored history
+
+  // this thread's disc, and its share of the block's pairs: those with discs of
+  // other blocks, and of a pair inside the block the lower disc's slot
+  V4<T> p{}, v{};
+  float2 rem = make_float2(0.0f, 0.0f);
+  int cnt = 0;
+  unsigned mask0 = 0u;
+  const unsigned* nbr = B.nbr[lp];
+  auto partner = [&](int s) { return slot_partner(B.head[lp][i], nbr, (size_t)n, i, s); };
+  const bool cut = (ctl->status & kStatusCapacity) != 0;  // a list overflowed: disc j may not list this one
+  auto lists = [&](int j) {
+    const uint4 h = B.head[lp][j];
+    const int c = (int)(h.x & 0xFFu);
+    for (int s = 0; s < c; ++s)
+      if (slot_partner(h, nbr, (size_t)n, j, s) == i) return true;
+    return false;
+  };
+  auto inside = [&](int j) { return (unsigned)(j - i0) < (unsigned)mine; };
+  unsigned yes = 0u;  // slots this block evaluates under this disc
+  if (own) {
+    const unsigned word = B.head[lp][i].x;
+    cnt = (int)(word & 0xFFu);
+    mask0 = word >> 8;
+    if (sizeof(T) == 4 && P.prem) rem = B.prem[lp][i];
+    p = B.pos[sp][i];
+    v = B.vel[sp][i];
+    spos[t] = p;
+    svel[t] = v;
+    for (int s = 0; s < cnt; ++s) {
+      const int j = partner(s);
+      if (!inside(j) || i < j || (cut && !lists(j))) yes |= 1u << s;
+    }
+  }
+  unsigned total;
+  const unsigned before = block_prefix((unsigned)__popc(yes), s_warp, total);
+  const int nc = (int)total;
+  const bool direct = nc > mc;  // no room: the discs' threads work on the global arrays
+  if (own && !direct) {
+    int e = (int)before;
+    base[t] = e;
+    for (int s = 0; s < cnt; ++s) {
+      if (!((yes >> s) & 1u)) continue;
+      const int j = partner(s);
+      const bool stored = (mask0 >> s) & 1u;
+      desc[e] = make_uint2((unsigned)t | (inside(j) ? (unsigned)(j - i0) << 16 : kOutside << 16), (unsigned)j);
+      hist[e] = stored ? B.hist[lp][(size_t)s * n + i] : V2<T>{T(0), T(0)};
+      on[e] = stored ? 2 : 0;
+      place[s * pb + t] = (unsigned short)((unsigned)e | (i < j ? kPlaceOwner : 0u));
+      ++e;
+    }
+    if (t == mine - 1) base[mine] = nc;
+  }
+  __syncthreads();
+  if (own && !direct) {
+    for (int s = 0; s < cnt; ++s) {
+      if ((yes >> s) & 1u) continue;
+      const int o = partner(s) - i0;
+      int e = base[o];
+      while (e < base[o + 1] - 1 && (int)desc[e].y != i) ++e;
+      place[s * pb + t] = (unsigned short)e;
+    }
+  }
+  // ledger partials of this warp's 32 discs (slot i / 32), carried in lane 0
+  const size_t gw = (size_t)i >> 5;
+  const bool books = lane == 0 && own;
+  double acc_diss = books ? B.diss_part[gw] : 0.0;
+  int k3 = 0;  // shared-memory reduction slot of the step
+  bool late = false;
+  unsigned bad = 0u;
+  int rebuild = 0;
+  __syncthreads();
+  while (true) {
+    const int primed = eval > 0 ? 1 : 0;
+    const int k1 = k3 == 2 ? 0 : k3 + 1;
+    if (!direct) {
+      const V4<T>* gpos = B.pos[sp];
+      const V4<T>* gvel = B.vel[sp];
+      auto law = [&](int e, const uint2& d, bool in, const V4<T>& x, const V4<T>& y) {
+        const int s = (int)(d.x & 0xFFFFu), o = (int)(d.x >> 16);
+        const bool owner = i0 + s < (int)d.y;
+        const V4<T> vx = svel[s], vy = in ? svel[o] : gvel[d.y];
+        const V4<T>& a = owner ? x : y;
+        const V4<T>& b = owner ? y : x;
+        const Geo<T> g = pair_geo<T>(P, a, b);
+        const V2<T> xi0 = (on[e] & 2) ? hist[e] : V2<T>{T(0), T(0)};
+        const PairOut<T> r = pair_force<T>(P, g, a, owner ? vx : vy, b, owner ? vy : vx, xi0);
+        hist[e] = r.xi;
+        on[e] = (r.xi.x != T(0)) || (r.xi.y != T(0)) ? 3 : 1;
+        res[e] = V4<T>{r.fx, r.fy, r.cr, r.diss};
+      };
+      // A thread per pair. FP64, whose pipe bounds the law, first lists the pairs
+      // that touch and evaluates them on full warps (82 -> 66 us a step at 65,535
+      // discs); in FP32 the list costs more than the idle lanes do (5% at 50,071).
+      constexpr bool LIST = sizeof(T) == 8;
+      for (int e0 = 0; e0 < nc; e0 += nt) {
+        const int e = e0 + t;
+        bool hit = false;
+        if (e < nc) {
+          const uint2 d = desc[e];
+          const int s = (int)(d.x & 0xFFFFu), o = (int)(d.x >> 16);
+          const bool in = LOCAL || o != (int)kOutside;
+          const V4<T> x = spos[s], y = in ? spos[o] : gpos[d.y];
+          const Geo<T> g = slot_geo<T>(P, i0 + s, (int)d.y, x, y);
+          hit = g.d2 < g.rs * g.rs;
+          if (!hit)
+            on[e] = 0;  // contact opened: reset
+          else if (!LIST)
+            law(e, d, in, x, y);
+        }
+        if (LIST) {
+          const unsigned hits = __ballot_sync(0xffffffffu, hit);
+          if (hits) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&s_touch[k3], __popc(hits));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (hit) touch[at + __popc(hits & ((1u << lane) - 1u))] = (unsigned short)e;
+          }
+        }
+      }
+      __syncthreads();
+      if (LIST) {
+        const int hits = s_touch[k3];
+        for (int w = t; w < hits; w += nt) {
+          const int e = touch[w];
+          const uint2 d = desc[e];
+          const int o = (int)(d.x >> 16);
+          const bool in = LOCAL || o != (int)kOutside;
+          law(e, d, in, spos[d.x & 0xFFFFu], in ? spos[o] : gpos[d.y]);
+        }
+        if (hits) __syncthreads();
+      }
+    }
+    if (sizeof(T) == 8 && t == 0) s_touch[k1] = 0;  // the next step's count: last read a step ago
+    // a disc's sums in slot order, its walls, and its move
+    ThreadLedger<T> L;
+    if (own) {
+      if (direct) {
+        ThreadLedger<T> D;  // (its address is taken: L itself stays in registers)
+        direct_disc<T>(P, B, sp, lp, i, primed, eval, D);
+        L = D;
+      } else {
+        // (the big build has no registers to keep the state in)
+        const V4<T> p0 = BIG ? spos[t] : p, v0 = BIG ? svel[t] : v;
+        Acc<T> fx, fy, tq;
+        for (int s = 0; s < cnt; ++s) {
+          const unsigned at = place[s * pb + t], e = at & ~kPlaceOwner;
+          if (!(on[e] & 1)) continue;
+          const V4<T> r = res[e];
+          if (at & kPlaceOwner) {
+            fx.add(r.x);
+            fy.add(r.y);
+            L.diss += r.w;
+          } else {
+            fx.add(-r.x);
+            fy.add(-r.y);
+          }
+          tq.add(p0.z * r.z);
+        }
+        wall_contacts<T, MODE>(P, B.whist[lp], i, p0, v0, fx, fy, tq, L, primed);
+        const T Fx = fx.get(), Fy = fy.get(), Tz = tq.get();
+        const T inv_m = v0.w;
+        const bool free = inv_m > T(0);
+        const T ax = free ? Fx * inv_m + P.gx : T(0);
+        const T ay = free ? Fy * inv_m + P.gy : T(0);
+        const T inv_i = inv_m * P.kinv / (p0.z * p0.z);
+        const T al = Tz * inv_i;
+        const Moved<T> m = move_particle<T, MODE>(P, p0, v0, rem, ax, ay, al, primed, L);
+        if (!BIG) {
+          p = m.pos;
+          v = m.vel;
+        }
+        rem = m.rem;
+        spos[t] = m.pos;
+        svel[t] = m.vel;
+        if (!LOCAL) {
+          B.pos[sp ^ 1][i] = m.pos;
+          B.vel[sp ^ 1][i] = m.vel;
+        }
+      }
+    }
+    // the warp's ledger partials (most warps have none)
+    const unsigned wbits = __reduce_max_sync(0xffffffffu, __float_as_uint(L.vmax2));
+    const bool wbad = __any_sync(0xffffffffu, L.bad);
+    if (lane == 0) {
+      if (wbits) atomicMax(&s_vmax[k3], wbits);
+      if (wbad) s_bad[k3] = 1;
+    }
+    if (__any_sync(0xffffffffu, L.diss != T(0))) {
+      T x = L.diss;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+      acc_diss += (double)x;
+    }
+    unsigned vbits;
+    if (t == 0) {  // the next step's slots: last read a step ago
+      s_vmax[k1] = 0u;
+      s_bad[k1] = 0;
+    }
+    if (LOCAL) {
+      __syncthreads();
+      vbits = s_vmax[k3];
+      bad = (unsigned)s_bad[k3];
+    } else {
+      grid_barrier(ctl, gridDim.x, epoch, &s_vmax[k3], &s_bad[k3], P.wait_budget, s_out);
+      ++epoch;
+      if (s_out[3]) {
+        late = true;
+        break;
+      }
+      vbits = s_out[1];
+      bad = s_out[2];
+    }
+    k3 = k1;
+    sp ^= 1;
+    ++eval;
+    disp += sqrtf(__uint_as_float(vbits)) * (float)P.dt;
+    rebuild = disp > P.rebuild_disp ? 1 : 0;
+    if (rebuild || bad || eval >= target) break;
+  }
+  if (late) {  // a barrier ran out of time: the state is not usable
+    if (t == 0 && (use_cond & 2)) cudaGraphSetConditional(h_loop, 0u);
+    return;
+  }
+  // write back what stayed on the chip
+  if (own && !direct) {
+    if (LOCAL) {
+      B.pos[sp][i] = p;
+      B.vel[sp][i] = v;
+    }
+    if (sizeof(T) == 4 && P.prem) B.prem[lp][i] = rem;
+    unsigned mask = 0u;
+    for (int s = 0; s < cnt; ++s) {
+      const unsigned e = place[s * pb + t] & ~kPlaceOwner;
+      const bool stored = (on[e] & 2) != 0;
+      if (stored) mask |= 1u << s;
+      if (stored || ((mask0 >> s) & 1u))
+        B.hist[lp][(size_t)s * n + i] = stored ? hist[e] : V2<T>{T(0), T(0)};
+    }
+    if (mask != mask0) B.head[lp][i].x = (unsigned)cnt | (mask << 8);
+  }
+  if (books) B.diss_part[gw] = acc_diss;
+  if (blockIdx.x == 0 && t == 0) {
+    ctl->sp = sp;
+    ctl->evals = eval;
+    ctl->disp = disp;
+    ctl->epoch = epoch;
+    ctl->rebuild_pending = rebuild;
+    if (bad) atomicOr(&ctl->status, (int)kStatusNonfinite);
+    const int keep_going = eval < target && !bad;
+    if (use_cond & 1) cudaGraphSetConditional(h_rebuild, (unsigned)rebuild);
+    if (use_cond & 2) cudaGraphSetConditional(h_loop, (unsigned)keep_going);
+  }
+}
+
+// A thread per disc: it keeps the disc's state in registers and its partner
+// indices, contact history and bond slots in shared memory, and evaluates its
+// bonds and candidates itself. For engines with bonds or an indenter (dealing
+// each bond once to the block's threads was no faster, and a bond's two sides
+// round differently in the one-step kernels, so it also changed the results'
+// last bits), and for dilute ones.
+template <class T, bool FEAT, bool LOCAL, bool BIG>
+__device__ __forceinline__ void run_discs(const Params<T>& P, const Bufs<T>& B, unsigned char* run_smem,
+                                          cudaGraphConditionalHandle h_rebuild, cudaGraphConditionalHandle h_loop,
+                                          int use_cond, int pb) {
+  constexpr int MODE = kBatch;  // the first evaluation of a state primes it
   __shared__ unsigned s_vmax[3], s_out[4];
   __shared__ int s_bad[3];
   Ctl* ctl = B.ctl;
@@ -72,10 +402,6 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
   const long long target = ctl->target;
   float disp = ctl->disp;
   unsigned epoch = ctl->epoch;
-  if (ctl->status & (kStatusNonfinite | kStatusTimeout)) {  // nothing to do with such a state
-    if (blockIdx.x == 0 && t == 0 && (use_cond & 2)) cudaGraphSetConditional(h_loop, 0u);
-    return;
-  }
   if (t < 3) {
     s_vmax[t] = 0u;
     s_bad[t] = 0;
@@ -391,6 +717,23 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
   }
 }
 
+template <class T, bool FEAT, bool LOCAL, bool BIG>
+__global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
+    force_kernel_run(Params<T> P, Bufs<T> B, cudaGraphConditionalHandle h_rebuild, cudaGraphConditionalHandle h_loop,
+                     int use_cond, int pb, int mc) {
+  extern __shared__ __align__(16) unsigned char run_smem[];
+  if (B.ctl->status & (kStatusNonfinite | kStatusTimeout)) {  // nothing to do with such a state
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (use_cond & 2)) cudaGraphSetConditional(h_loop, 0u);
+    return;
+  }
+  // from one candidate pair per disc on, pairs pay for their barrier (FP32, us a
+  // step, discs / pairs: 50,071 touching discs 8.6 / 7.1, 90,000 dilute ones 4.3 / 5.6)
+  if (!FEAT && B.ctl->candidates >= 2ll * P.n)
+    run_pairs<T, LOCAL, BIG>(P, B, run_smem, h_rebuild, h_loop, use_cond, pb, mc);
+  else
+    run_discs<T, FEAT, LOCAL, BIG>(P, B, run_smem, h_rebuild, h_loop, use_cond, pb);
+}
+
 // Resident form of the pipelined step (FP32), for engines of many discs per
 // thread: the one-step kernel's pass over the discs, with a grid barrier in the
 // place of the launch. At 1,048,576 discs the launch, its ramp and its last
@@ -403,7 +746,7 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
 template <class T, int BLOCK, bool FEAT, bool CHUNKED>
 __global__ void __launch_bounds__(BLOCK, 1)
     force_kernel_run_async(Params<T> P, Bufs<T> B, cudaGraphConditionalHandle h_rebuild,
-                           cudaGraphConditionalHandle h_loop, int use_cond, int) {
+                           cudaGraphConditionalHandle h_loop, int use_cond, int, int) {
   extern __shared__ __align__(16) unsigned char run_smem[];
   __shared__ unsigned s_vmax[3], s_out[4];
   __shared__ int s_bad[3];

@@ -2,22 +2,30 @@
 // advances many steps, with a grid barrier in the place of the kernel boundary.
 //
 // What bounds a small or middle-sized engine is not bandwidth but the chain of
-// one step: in the step graph a WHILE iteration costs 3.9 us with an empty
-// body, and a step of 3,249 discs took 11 us. Here each thread owns one disc
-// for the whole launch: its state, list head and remainder stay in registers,
-// its partner indices, contact history and bond slots in shared memory, and
-// only the positions and velocities that partners read go through L2. A grid
-// barrier (one arrival per block, one 16-byte poll that also returns the
-// speed bound and the error flag) costs 1.2 us on 152 blocks. An engine that
-// fits one block keeps the positions in shared memory too and needs only the
-// block's own barrier.
+// one step. In the step graph a WHILE iteration costs 3.9 us with an empty body
+// (a step of 3,249 discs took 11 us). Here a block owns a contiguous range of
+// sorted discs for the whole launch, and a grid barrier (one arrival per block,
+// one 16-byte poll that also returns the speed bound and the error flag) costs
+// 1.2 us on 152 blocks; an engine of one block needs none. Only positions and
+// velocities that other blocks read go through L2. Two ways through a step:
 //
-// Measured (GB300, a pass of upload, n steps, read-back; before -> now):
-// 300 touching discs x 100 steps 1,924 -> 950 us, 3,249 dilute discs x 200
-// steps 2,405 -> 814 us (11 -> 3.4 us a step), 50,071 touching discs x 100
-// steps 1,822 -> 954 us, a 2,328-disc bonded sheet x 200 steps 5,083 -> 2,620
-// us, 65,535 touching discs in FP64 x 50 steps 7,618 -> 6,486 us (bound by the
-// FP64 pipe, not by the chain).
+// A thread per disc keeps the disc's state in registers and its partner indices,
+// history and bond slots in shared memory, and evaluates its bonds and
+// candidates one after another.
+//
+// A thread per pair (no bonds, a candidate pair per disc or more): each pair of
+// the block is evaluated once, also when both discs are the block's, by any of
+// its threads; a disc's thread then sums the results in slot order. At this
+// occupancy a contact law is a chain of 0.4 us, and a disc of a bed has six
+// candidates; in FP64 the pipe (two lanes a clock) bounds the law itself.
+//
+// Measured (GB300, a pass of upload where it says so, n steps, read-back):
+//                                              one-step  per disc  per pair
+//   300 touching discs x 100 steps, upload        1,924       950       713 us
+//   3,249 dilute discs x 200 steps, upload        2,405       814       852
+//   50,071 touching discs x 100 steps             1,822       954       835
+//   65,535 touching discs x 50 steps, FP64        7,618     6,486     3,938
+//   2,328-disc bonded sheet x 200 steps, upload   5,083     2,620         -
 //
 // The launch ends when the list must be rebuilt, the step target is reached or
 // the state went non-finite; the step graph loops around it. Every disc is
@@ -84,9 +92,8 @@ struct PlainFetch {
 };
 
 // Threads per block, in two builds: `big` halves the registers of a thread for
-// engines that need every thread of the chip. Without spills the bond, FP64
-// and three-candidates-in-flight code takes up to 255 registers, FP32 contacts
-// 128; the big builds take their candidates one at a time.
+// engines that need every thread of the chip. Without spills bonds and FP64
+// take up to 255 registers, FP32 contacts 128.
 template <class T>
 constexpr int run_block(bool feat, bool big) {
   return (sizeof(T) == 4 && !feat ? 512 : 256) * (big ? 2 : 1);
@@ -98,7 +105,40 @@ constexpr int kRunDiscs = 128;
 constexpr int kRunLocal = 512;
 constexpr int kRunLocalBonds = 128;
 
-// Shared memory of a block that owns `pb` discs: byte offsets.
+// Shared memory of a block without bonds that owns `pb` discs and has room for
+// mc pairs: byte offsets. kRunPairs: pairs per disc it must have room for (a
+// hexagonal bed evaluates 3.4 per disc of a 128-disc block, 3.2 of a 352-disc
+// one); a block with more works on the global arrays.
+constexpr int kRunPairs = 4;
+
+struct PairLayout {
+  size_t pos, vel, res, hist, desc, base, place, touch, on, total;
+};
+
+template <class T>
+__host__ __device__ inline PairLayout pair_layout(int W, int pb, int mc) {
+  PairLayout L;
+  size_t o = 0;
+  const size_t b = (size_t)pb, c = (size_t)mc;
+  auto take = [&](size_t bytes) {
+    const size_t at = o;
+    o += (bytes + 15) & ~size_t(15);
+    return at;
+  };
+  L.pos = take(b * sizeof(V4<T>));
+  L.vel = take(b * sizeof(V4<T>));
+  L.res = take(c * sizeof(V4<T>));
+  L.hist = take(c * sizeof(V2<T>));
+  L.desc = take(c * 8);
+  L.base = take((b + 1) * 4);
+  L.place = take((size_t)W * b * 2);
+  L.touch = take(c * 2);
+  L.on = take(c);
+  L.total = o;
+  return L;
+}
+
+// Shared memory of a block with bonds that owns `pb` discs: byte offsets.
 struct RunLayout {
   size_t pos, vel, strain, hist, bref, bus, bstr, tail, bpart, bfail, total;
 };
@@ -138,7 +178,7 @@ __host__ __device__ inline RunLayout run_layout(int W, int BM, int pb, int local
 // block with its positions in shared memory (local) or over a cooperative grid
 // (of big blocks).
 template <class T>
-using RunFn = void (*)(Params<T>, Bufs<T>, cudaGraphConditionalHandle, cudaGraphConditionalHandle, int, int);
+using RunFn = void (*)(Params<T>, Bufs<T>, cudaGraphConditionalHandle, cudaGraphConditionalHandle, int, int, int);
 template <class T>
 RunFn<T> run_fn(bool feat, bool local, bool big);
 

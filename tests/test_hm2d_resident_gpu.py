@@ -49,18 +49,20 @@ def _same(a, b, bonded):
     return la
 
 
-# 4 and 484 discs: one block; 529: the first grid; 3249: a partial last block;
-# 80089: the big build (FP64: too large); 160000: too large for one disc per thread
+# 4 and 484 discs: one block; 529: the first grid; 3249: a partial last block; 80089: the big
+# build (FP64: too large); 160000: more discs than threads. The narrow skin leaves under one
+# candidate pair per disc (a thread per disc), the wide one more (a thread per pair).
+@pytest.mark.parametrize("skin", [0.02e-3, 0.5e-3])
 @pytest.mark.parametrize("precision,side", [(32, 2), (32, 22), (32, 23), (32, 57), (32, 283), (32, 400),
                                             (64, 16), (64, 33), (64, 205), (64, 283)])
-def test_granular_resident_steps_equal_one_step_launches(hm, precision, side):
-    cfg, st = dense_gas(side, seed=side, precision=precision)
+def test_granular_resident_steps_equal_one_step_launches(hm, precision, side, skin):
+    cfg, st = dense_gas(side, seed=side, precision=precision, skin=skin)
     blocks = (1, 2, 1, 60)
     a = _run(hm, cfg, st, None, True, blocks)
     led = _same(a, _run(hm, cfg, st, None, False, blocks), False)
     assert led["evals"] == 64 and led["status"] == 0
     if side >= 22:
-        assert led["rebuilds"] >= 2 and led["dissipated"] > 0.0
+        assert led["dissipated"] > 0.0 and (led["rebuilds"] >= 2 or skin > 0.1e-3)
 
 
 # 90 and 128 discs: one block; 182: the first grid; 40000: the big build (FP64 too)
@@ -72,6 +74,16 @@ def test_bonded_resident_steps_equal_one_step_launches(hm, precision, nx, ny):
     a = _run(hm, cfg, st, (bonds, strength), True, blocks)
     led = _same(a, _run(hm, cfg, st, (bonds, strength), False, blocks), True)
     assert led["evals"] == 200 and led["tool_work"] > 0.0
+
+
+# wide skins: more pairs per disc than a block's shared memory holds, so its threads work on
+# the global arrays (FP32 and FP64 big builds)
+@pytest.mark.parametrize("precision,side,skin,slots", [(32, 390, 2.0e-3, 24), (64, 277, 2.5e-3, 24)])
+def test_blocks_without_room_for_their_pairs(hm, precision, side, skin, slots):
+    cfg, st = dense_gas(side, seed=side, precision=precision, skin=skin, max_neighbors=slots)
+    a = _run(hm, cfg, st, None, True, (25,))
+    led = _same(a, _run(hm, cfg, st, None, False, (25,)), False)
+    assert led["status"] == 0 and led["dissipated"] > 0.0
 
 
 def test_indenter_without_bonds(hm):
