@@ -446,8 +446,7 @@ struct Engine final : EngineBase {
         (rc = alloc(&B.cell_fill, (size_t)P.nkeys)) || (rc = alloc(&B.perm, n)) ||
         (rc = alloc(&B.block_sums, (size_t)scan_blocks)) || (rc = alloc(&B.tmp_cell, n)) ||
         (rc = alloc(&B.tmp_off, n)) || (rc = alloc(&B.diss_part, (size_t)nwarp_slots)) ||
-        (rc = alloc(&B.peek_part, (size_t)nblocks * 12)) || (rc = alloc(&B.peek_vel, n)) ||
-        (rc = alloc(&B.peek_force, n)) || (rc = alloc(&B.ctl, 1)) || (rc = alloc(&B.invperm, n)) ||
+        (rc = alloc(&B.peek_part, (size_t)nblocks * 12)) || (rc = alloc(&B.ctl, 1)) || (rc = alloc(&B.invperm, n)) ||
         (rc = alloc(&B.frac_part, (size_t)nwarp_slots)) || (rc = alloc(&B.ind_part, 8 * (size_t)nwarp_slots)) ||
         (rc = alloc(&B.load, 2 * (size_t)std::max(P.load_cap, 1))))
       return rc;
@@ -801,26 +800,32 @@ struct Engine final : EngineBase {
     return TDEM_OK;
   }
 
+  void launch_read(double* pos, double* vel, double* omega, double* force, double* torque, cudaStream_t s) {
+    const int pr = primed ? 1 : 0;
+    auto fn = sum64 ? (feat() ? &read_kernel<T, true, true> : &read_kernel<T, false, true>)
+                    : (feat() ? &read_kernel<T, true, false> : &read_kernel<T, false, false>);
+    fn<<<grid_n(), kThreads, 0, s>>>(P, B, pr, pos, vel, omega, force, torque);
+  }
+
   int read_state(double* pos, double* vel, double* omega, double* force, double* torque, int host,
                  cudaStream_t s) override {
     if (!has_state) return tdem::fail(&err, TDEM_ERR_STATE, "read before set_state");
-    int rc = peek(s);
-    if (rc) return rc;
+    launch_strain(s);
     const size_t n = (size_t)P.n;
     if (host) {
-      double* d = stage;  // pos 2n, vel 2n, omega n, force 2n, torque n
-      unpack_kernel<T><<<grid_n(), kThreads, 0, s>>>(P, B, d, d + 2 * n, d + 4 * n, d + 5 * n, d + 7 * n);
+      double* d = stage;  // pos 2n, vel 2n, force 2n, omega n, torque n
+      launch_read(d, d + 2 * n, d + 6 * n, d + 4 * n, d + 7 * n, s);
       TDEM_CUDA_TRY(&err, cudaGetLastError());
       TDEM_CUDA_TRY(&err, cudaMemcpyAsync(host_stage, stage, 8 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
       TDEM_CUDA_TRY(&err, cudaStreamSynchronize(s));
       if (pos) tdem::parallel_copy(pos, host_stage, 2 * n * sizeof(double));
       if (vel) tdem::parallel_copy(vel, host_stage + 2 * n, 2 * n * sizeof(double));
-      if (omega) tdem::parallel_copy(omega, host_stage + 4 * n, n * sizeof(double));
-      if (force) tdem::parallel_copy(force, host_stage + 5 * n, 2 * n * sizeof(double));
+      if (omega) tdem::parallel_copy(omega, host_stage + 6 * n, n * sizeof(double));
+      if (force) tdem::parallel_copy(force, host_stage + 4 * n, 2 * n * sizeof(double));
       if (torque) tdem::parallel_copy(torque, host_stage + 7 * n, n * sizeof(double));
       return TDEM_OK;
     }
-    unpack_kernel<T><<<grid_n(), kThreads, 0, s>>>(P, B, pos, vel, omega, force, torque);
+    launch_read(pos, vel, omega, force, torque, s);
     TDEM_CUDA_TRY(&err, cudaGetLastError());
     return TDEM_OK;
   }
@@ -1555,9 +1560,6 @@ int tdem_hm_contact_forces_noalloc(const tdem_hm_config* cfg, const double* pos,
   B.tmp_cell = c.take<int>(n);
   B.tmp_off = c.take<V2<float>>(n);
   B.diss_part = c.take<double>((size_t)nb * (kThreads / 32));
-  B.peek_part = c.take<double>((size_t)nb * 12);
-  B.peek_vel = c.take<V4<float>>(n);
-  B.peek_force = c.take<V4<float>>(n);
   B.invperm = c.take<int>(n);
   B.ctl = c.take<Ctl>(1);
   int* status_dev = c.take<int>(1);
@@ -1570,8 +1572,7 @@ int tdem_hm_contact_forces_noalloc(const tdem_hm_config* cfg, const double* pos,
                                                                                B.cell_fill, P.nkeys);
   pack_kernel<float><<<nb, kThreads, 0, s>>>(P, B, pos, vel, omega, radius, mass, inertia);
   launch_rebuild_seq<float>(P, B, s);
-  force_kernel<float, kPeek, false><<<nb, kThreads, 0, s>>>(P, B, 0, 0, 0, 0, StepHint{});
-  unpack_kernel<float><<<nb, kThreads, 0, s>>>(P, B, nullptr, nullptr, nullptr, out_force, out_torque);
+  read_kernel<float, false, false><<<nb, kThreads, 0, s>>>(P, B, 0, nullptr, nullptr, nullptr, out_force, out_torque);
   noalloc_status_kernel<<<1, 1, 0, s>>>(B.ctl, status_dev);
   cudaError_t e = cudaGetLastError();
   int status = 0;

@@ -183,8 +183,8 @@ struct Bufs {
   // ledger and read-back
   double* diss_part;   // per step-kernel warp: committed dissipation (J)
   double* peek_part;   // per block x 8: kinetic, potential, Hertz, tangential, dissipation
-  V4<T>* peek_vel;     // integer-time velocity (vx, vy, omega, -)
-  V4<T>* peek_force;   // integer-time force (fx, fy, torque, -)
+  V4<T>* peek_vel;     // batched engine: integer-time velocity (vx, vy, omega, -)
+  V4<T>* peek_force;   // batched engine: integer-time force (fx, fy, torque, -)
   Ctl* ctl;
   // bonded-particle model
   unsigned* bpart[2];
