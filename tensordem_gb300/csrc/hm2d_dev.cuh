@@ -254,12 +254,16 @@ struct WindowFetch {
   __device__ __forceinline__ V4<T> v(int j) const { return in(j) ? svel[(j - off) & mask] : vel[j]; }
 };
 
-// The geometry of particle i's candidate j at position q, from canonically
-// ordered operands; the pair touches when d2 < rs^2.
+// The geometry of particle i's candidate j at position q; the pair touches
+// when d2 < rs^2. Formed from i to j and turned into the canonical direction:
+// differences, their fused sum and rs are the same numbers either way (negation
+// is exact), and the test needs no selection of its operands.
 template <class T>
-__device__ __forceinline__ Geo<T> slot_geo(const Params<T>& P, int i, int j, const V4<T>& p, const V4<T>& q) {
-  const bool owner = i < j;
-  return pair_geo<T>(P, owner ? p : q, owner ? q : p);
+__device__ __forceinline__ void canonical(Geo<T>& g, bool owner) {
+  if (!owner) {
+    g.dx = -g.dx;
+    g.dy = -g.dy;
+  }
 }
 
 // A touching candidate slot s of particle i, its operands loaded: partner
@@ -304,12 +308,13 @@ __device__ __forceinline__ void do_slot(const Params<T>& P, const F& fetch,
                                         unsigned& nmask, A& fx, A& fy, A& tq, T& diss, T& un,
                                         T& ut, int primed) {
   constexpr bool COMMIT = kCommits<MODE>;
-  const Geo<T> g = slot_geo<T>(P, i, j, p, q);
+  Geo<T> g = pair_geo<T>(P, p, q);
   const bool stored = (mask >> s) & 1u;
   if (!(g.d2 < g.rs * g.rs)) {
     if (COMMIT && stored) hist[slot] = V2<T>{T(0), T(0)};  // contact opened: reset
     return;
   }
+  canonical<T>(g, i < j);
   const V4<T> w = fetch.v(j);
   const V2<T> xi0 = stored ? hist[slot] : V2<T>{T(0), T(0)};
   touching_slot<T, MODE>(P, hist + slot, i, j, s, g, p, v, q, w, xi0, stored, nmask, fx, fy, tq, diss, un, ut, primed);
@@ -945,10 +950,10 @@ __device__ __forceinline__ void process_particle_q(const Params<T>& P, const Buf
   const T Fx = fx.get(), Fy = fy.get(), Tz = tq.get();
   const T inv_m = v.w;  // 0 for a clamped disc
   const bool free = inv_m > T(0);
-  const T inv_i = inv_m * P.kinv / (p.z * p.z);
   const T ax = free ? Fx * inv_m + P.gx : T(0);
   const T ay = free ? Fy * inv_m + P.gy : T(0);
-  const T al = Tz * inv_i;
+  T al = Tz;
+  if (Tz != T(0)) al = Tz * (inv_m * P.kinv / (p.z * p.z));  // few discs of a dilute engine: spare the division
   if (!kCommits<MODE>) {
     const T h = primed ? P.half_dt : T(0);
     const T vx = v.x + h * ax, vy = v.y + h * ay, om = v.z + h * al;

@@ -226,7 +226,7 @@ __device__ __forceinline__ void run_pairs(const Params<T>& P, const Bufs<T>& B, 
           const int s = (int)(d.x & 0xFFFFu), o = (int)(d.x >> 16);
           const bool in = LOCAL || o != (int)kOutside;
           const V4<T> x = spos[s], y = in ? spos[o] : gpos[d.y];
-          const Geo<T> g = slot_geo<T>(P, i0 + s, (int)d.y, x, y);
+          const Geo<T> g = pair_geo<T>(P, x, y);
           hit = g.d2 < g.rs * g.rs;
           if (!hit)
             on[e] = 0;  // contact opened: reset
@@ -288,8 +288,8 @@ __device__ __forceinline__ void run_pairs(const Params<T>& P, const Bufs<T>& B, 
         const bool free = inv_m > T(0);
         const T ax = free ? Fx * inv_m + P.gx : T(0);
         const T ay = free ? Fy * inv_m + P.gy : T(0);
-        const T inv_i = inv_m * P.kinv / (p0.z * p0.z);
-        const T al = Tz * inv_i;
+        T al = Tz;
+        if (Tz != T(0)) al = Tz * (inv_m * P.kinv / (p0.z * p0.z));
         const Moved<T> m = move_particle<T, MODE>(P, p0, v0, rem, ax, ay, al, primed, L);
         if (!BIG) {
           p = m.pos;
@@ -562,9 +562,10 @@ __device__ __forceinline__ void run_discs(const Params<T>& P, const Bufs<T>& B, 
 #pragma unroll
         for (int u = 0; u < KS; ++u) {
           if (on[u]) {
-            g[u] = slot_geo<T>(P, i, j[u], p, q[u]);
+            g[u] = pair_geo<T>(P, p, q[u]);
             on[u] = g[u].d2 < g[u].rs * g[u].rs;
             if (on[u]) w[u] = fetch.v(j[u]);
+            canonical<T>(g[u], i < j[u]);
           }
         }
 #pragma unroll
@@ -585,10 +586,10 @@ __device__ __forceinline__ void run_discs(const Params<T>& P, const Bufs<T>& B, 
       const T Fx = fx.get(), Fy = fy.get(), Tz = tq.get();
       const T inv_m = v.w;
       const bool free = inv_m > T(0);
-      const T inv_i = inv_m * P.kinv / (p.z * p.z);
       const T ax = free ? Fx * inv_m + P.gx : T(0);
       const T ay = free ? Fy * inv_m + P.gy : T(0);
-      const T al = Tz * inv_i;
+      T al = Tz;
+      if (Tz != T(0)) al = Tz * (inv_m * P.kinv / (p.z * p.z));
       const Moved<T> m = move_particle<T, MODE>(P, p, v, rem, ax, ay, al, primed, L);
       p = m.pos;
       v = m.vel;
