@@ -86,6 +86,16 @@ def test_blocks_without_room_for_their_pairs(hm, precision, side, skin, slots):
     assert led["status"] == 0 and led["dissipated"] > 0.0
 
 
+# pairs per disc of a block (2.0, 3.6 and 4.0, and those that two blocks evaluate) on both sides
+# of the two thirds of its room (6.2) up to which FP64 pairs keep their effective radius and mass
+@pytest.mark.parametrize("skin", [0.5e-3, 1.0e-3, 1.5e-3])
+def test_fp64_pairs_with_and_without_room_for_their_constants(hm, skin):
+    cfg, st = dense_gas(270, seed=270, precision=64, skin=skin, max_neighbors=24)
+    a = _run(hm, cfg, st, None, True, (1, 40))
+    led = _same(a, _run(hm, cfg, st, None, False, (1, 40)), False)
+    assert led["status"] == 0 and led["dissipated"] > 0.0
+
+
 def test_indenter_without_bonds(hm):
     """An engine with an indenter but no bond slots takes the bonded build with none."""
     from dataclasses import replace
