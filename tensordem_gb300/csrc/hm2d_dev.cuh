@@ -80,11 +80,10 @@ __device__ __forceinline__ PairOut<T> contact_law(const Params<T>& P, T delta, T
                                                   T rb, const V4<T>& va, const V4<T>& vb, V2<T> xi);
 
 // One active contact (g.d2 < g.rs^2): force on a, torque lever term, history.
-// effective(reff, meff): the pair's effective radius and mass.
-template <class T, class E>
+template <class T>
 __device__ __forceinline__ PairOut<T> pair_force(const Params<T>& P, const Geo<T>& g, const V4<T>& pa,
                                                  const V4<T>& va, const V4<T>& pb, const V4<T>& vb,
-                                                 V2<T> xi, E effective) {
+                                                 V2<T> xi) {
   if (!(va.w + vb.w > T(0))) {  // two clamped discs exchange no force
     PairOut<T> o;
     o.active = true;
@@ -103,17 +102,8 @@ __device__ __forceinline__ PairOut<T> pair_force(const Params<T>& P, const Geo<T
     nx = g.dx / d;
     ny = g.dy / d;
   }
-  effective(reff, meff);
+  pair_effective<T>(pa.z, pb.z, va.w, vb.w, reff, meff);
   return contact_law<T>(P, delta, nx, ny, reff, meff, pa.z, pb.z, va, vb, xi);
-}
-
-template <class T>
-__device__ __forceinline__ PairOut<T> pair_force(const Params<T>& P, const Geo<T>& g, const V4<T>& pa,
-                                                 const V4<T>& va, const V4<T>& pb, const V4<T>& vb,
-                                                 V2<T> xi) {
-  return pair_force<T>(P, g, pa, va, pb, vb, xi, [&](T& reff, T& meff) {
-    pair_effective<T>(pa.z, pb.z, va.w, vb.w, reff, meff);
-  });
 }
 
 // The contact law proper, from the overlap delta > 0 and the unit normal n

@@ -220,16 +220,21 @@ __device__ __forceinline__ void run_pairs(const Params<T>& P, const Bufs<T>& B, 
         const Geo<T> g = pair_geo<T>(P, a, b);
         const unsigned was = on[e];
         const V2<T> xi0 = (was & 2) ? hist[e] : V2<T>{T(0), T(0)};
-        const PairOut<T> r =
-            pair_force<T>(P, g, a, owner ? vx : vy, b, owner ? vy : vx, xi0, [&](T& reff, T& meff) {
-              if (KEEP && (was & 4)) {
-                reff = eff[e].x;
-                meff = eff[e].y;
-              } else {
-                pair_effective<T>(x.z, y.z, vx.w, vy.w, reff, meff);
-                if (KEEP && keep) eff[e] = V2<T>{reff, meff};
-              }
-            });
+        PairOut<T> r;
+        if (KEEP && vx.w + vy.w > T(0)) {  // pair_force with the constants kept
+          V2<T> c;
+          if (was & 4) {
+            c = eff[e];
+          } else {
+            pair_effective<T>(x.z, y.z, vx.w, vy.w, c.x, c.y);
+            if (keep) eff[e] = c;
+          }
+          const T d0 = dev_sqrt(g.d2);
+          r = contact_law<T>(P, g.rs - d0, g.dx / d0, g.dy / d0, c.x, c.y, a.z, b.z, owner ? vx : vy,
+                             owner ? vy : vx, xi0);
+        } else {
+          r = pair_force<T>(P, g, a, owner ? vx : vy, b, owner ? vy : vx, xi0);
+        }
         hist[e] = r.xi;
         on[e] = (unsigned char)(((r.xi.x != T(0)) || (r.xi.y != T(0)) ? 3 : 1) | (KEEP && keep ? 4 : 0));
         res[e] = V4<T>{r.fx, r.fy, r.cr, r.diss};
