@@ -20,7 +20,8 @@
 // one-step launches -> this): 32 runs of 100 to 2,000 discs (22,673 discs) x
 // 100 steps 10,268 -> 2,220 us (99 -> 20 us a step: 91 chunks of 8 tiles had
 // kept 91 of 4,864 warps busy); 256 runs of 100 to 20,000 discs (1.16M) x 40
-// steps 12,487 -> 7,080 us.
+// steps 12,487 -> 7,080 us (6,950 with the lean contact test; L2 prefetches of
+// the next tile's bond rows cost 9% of it).
 #include "batch_run.cuh"
 
 namespace tdem {

@@ -766,7 +766,8 @@ __global__ void __launch_bounds__(run_block<T>(FEAT, BIG), 1)
 // block cost 6 us of a 24 us step. Measured (GB300, steps and a state read):
 // 1,048,576 discs x 100 steps 2,894 -> 2,717 us, 4,194,304 discs x 40 steps
 // 6,708 -> 4,920 us (the default loop had been the one-thread-per-disc kernel),
-// the 1,048,576-disc bonded sheet x 40 steps 6,026 -> 5,605 us.
+// the 1,048,576-disc bonded sheet x 40 steps 6,026 -> 5,605 us; with read_kernel
+// and the lean contact test 2,425, 3,747 and 5,435 us.
 // CHUNKED: ledger partials per 32 sorted discs, as variant 0 books them; else
 // per warp of the grid, as the pipelined variants do.
 template <class T, int BLOCK, bool FEAT, bool CHUNKED>

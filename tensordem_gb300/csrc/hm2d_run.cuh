@@ -25,6 +25,7 @@
 //   3,249 dilute discs x 200 steps, upload        2,405       814       852
 //   50,071 touching discs x 100 steps             1,822       954       835
 //   65,535 touching discs x 50 steps, FP64        7,618     6,486     3,938
+//     (3,636 with each pair's effective radius and mass kept)
 //   2,328-disc bonded sheet x 200 steps, upload   5,083     2,620         -
 //
 // The launch ends when the list must be rebuilt, the step target is reached or
