@@ -191,9 +191,27 @@ __global__ void cc_out_kernel(Params<T> P, Bufs<T> B, const int* parent, const i
   if (i < P.n) out[B.orig[B.ctl->lp][i]] = label[parent[i]];
 }
 
+// Engines that rebuild in one block: where its passes over the discs cost less
+// than the launches of the general pipeline. Measured (GB300, us per rebuild, one
+// block / general): FP32 256 discs 17 / 59, 2,025 32 / 64, 4,096 52 / 63, 8,100
+// 94 / 64; FP64, whose search runs on one SM's FP64 pipe, 256 discs 37 / 78,
+// 3,249 254 / 77. A bonded disc gathers its slots too (2,328 discs lose 1% of a
+// solve). The keys are scanned and cleared by the block, hence their bound.
+constexpr long long kSmallRebuild = 4096;
+
+template <class T>
+bool small_rebuild(const Params<T>& P) {
+  const long long weight = (long long)(P.BMAX > 0 ? 4 : 1) * (sizeof(T) == 8 ? 8 : 1);
+  return P.n * weight <= kSmallRebuild && P.nkeys <= 4 * kSmallRebuild;
+}
+
 // The rebuild pipeline (every kernel a no-op unless ctl->rebuild_pending).
 template <class T>
 void launch_rebuild_seq(const Params<T>& P, const Bufs<T>& B, cudaStream_t s) {
+  if (small_rebuild(P)) {
+    rebuild_small_kernel<T><<<1, kScanThreads, 0, s>>>(P, B);
+    return;
+  }
   const int nb = (P.n + kThreads - 1) / kThreads;
   const int nk = (P.nkeys + kThreads - 1) / kThreads;
   const int sb = (P.nkeys + kScanChunk - 1) / kScanChunk;

@@ -1620,9 +1620,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) force_kernel_bulk(Params<T> P, Bu
 // instance, or of one that went non-finite during a step, take the dead key
 // (ctl->key_hi) and fall off the end of the sorted arrays.
 template <class T, bool MULTI = false>
-__global__ void bin_kernel(Params<T> P, Bufs<T> B) {
+__device__ __forceinline__ void bin_pass(const Params<T>& P, const Bufs<T>& B) {
   Ctl* ctl = B.ctl;
-  if (!ctl->rebuild_pending) return;
   const int sp = ctl->sp, lp = ctl->lp;
   const int n = MULTI ? ctl->n_old : P.n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1666,6 +1665,11 @@ __global__ void bin_kernel(Params<T> P, Bufs<T> B) {
     if (MULTI) B.tmp_key[i] = key;
     atomicAdd(&B.cell_count[key], 1);
   }
+}
+
+template <class T, bool MULTI = false>
+__global__ void bin_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending) bin_pass<T, MULTI>(P, B);
 }
 
 // 2. exclusive scan of the per-key counts (three phases, 4096 keys per block).
@@ -1757,9 +1761,8 @@ static __global__ void scan_add_kernel(const Ctl* ctl, int* out, const int* bloc
 
 // 3. scatter old indices into their key's range (order fixed by step 4)
 template <class T, bool MULTI = false>
-__global__ void scatter_kernel(Params<T> P, Bufs<T> B) {
+__device__ __forceinline__ void scatter_pass(const Params<T>& P, const Bufs<T>& B) {
   const Ctl* ctl = B.ctl;
-  if (!ctl->rebuild_pending) return;
   const int n = MULTI ? ctl->n_old : P.n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     int key;
@@ -1774,13 +1777,17 @@ __global__ void scatter_kernel(Params<T> P, Bufs<T> B) {
   }
 }
 
+template <class T, bool MULTI = false>
+__global__ void scatter_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending) scatter_pass<T, MULTI>(P, B);
+}
+
 // 4. deterministic order inside each cell: ascending original id (the
 // instance-local id in the batched engine; a cell never mixes instances).
 // The dead key is left unsorted.
 template <class T, bool MULTI = false>
-__global__ void cellsort_kernel(Params<T> P, Bufs<T> B) {
+__device__ __forceinline__ void cellsort_pass(const Params<T>& P, const Bufs<T>& B) {
   Ctl* ctl = B.ctl;
-  if (!ctl->rebuild_pending) return;
   const int nkeys = MULTI ? ctl->key_hi : P.nkeys;
   const int* orig = B.orig[ctl->lp];
   for (int key = blockIdx.x * blockDim.x + threadIdx.x; key < nkeys; key += gridDim.x * blockDim.x) {
@@ -1800,11 +1807,15 @@ __global__ void cellsort_kernel(Params<T> P, Bufs<T> B) {
   }
 }
 
+template <class T, bool MULTI = false>
+__global__ void cellsort_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending) cellsort_pass<T, MULTI>(P, B);
+}
+
 // 5. gather particle state into the new order (other buffers)
 template <class T, bool MULTI = false>
-__global__ void gather_kernel(Params<T> P, Bufs<T> B) {
+__device__ __forceinline__ void gather_pass(const Params<T>& P, const Bufs<T>& B) {
   Ctl* ctl = B.ctl;
-  if (!ctl->rebuild_pending) return;
   const int sp = ctl->sp, lp = ctl->lp;
   const int nn = MULTI ? ctl->n_live : P.n;  // MULTI: the live count after this rebuild
   const size_t n = (size_t)P.n;
@@ -1831,11 +1842,15 @@ __global__ void gather_kernel(Params<T> P, Bufs<T> B) {
   }
 }
 
+template <class T, bool MULTI = false>
+__global__ void gather_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending) gather_pass<T, MULTI>(P, B);
+}
+
 // 5b. bond slots follow their disc; partners are renamed to the new order
 template <class T, bool MULTI = false>
-__global__ void bond_gather_kernel(Params<T> P, Bufs<T> B) {
+__device__ __forceinline__ void bond_gather_pass(const Params<T>& P, const Bufs<T>& B) {
   Ctl* ctl = B.ctl;
-  if (!ctl->rebuild_pending || P.BMAX == 0) return;
   const int lp = ctl->lp;
   const int nn = MULTI ? ctl->n_live : P.n;
   const size_t n = (size_t)P.n;
@@ -1861,11 +1876,15 @@ __global__ void bond_gather_kernel(Params<T> P, Bufs<T> B) {
   }
 }
 
+template <class T, bool MULTI = false>
+__global__ void bond_gather_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending && P.BMAX > 0) bond_gather_pass<T, MULTI>(P, B);
+}
+
 // 6. candidate partners: the 3x3 cells around each particle, fixed order
 template <class T, bool MULTI = false>
-__global__ void build_nbr_kernel(Params<T> P, Bufs<T> B) {
+__device__ __forceinline__ void build_nbr_pass(const Params<T>& P, const Bufs<T>& B) {
   Ctl* ctl = B.ctl;
-  if (!ctl->rebuild_pending) return;
   const int sp1 = ctl->sp ^ 1, lp1 = ctl->lp ^ 1;
   const int nn = MULTI ? ctl->n_live : P.n;
   const V4<T>* pos = B.pos[sp1];
@@ -1928,14 +1947,18 @@ __global__ void build_nbr_kernel(Params<T> P, Bufs<T> B) {
   }
 }
 
+template <class T, bool MULTI = false>
+__global__ void build_nbr_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending) build_nbr_pass<T, MULTI>(P, B);
+}
+
 // 7. tangential-history remap keyed by the original-id pair: each particle
 // looks its new partner up in its own old list (old sorted indices through
 // perm) and carries the stored displacement over, flipping its sign when the
 // pair's lower sorted index changed sides.
 template <class T, bool MULTI = false>
-__global__ void link_kernel(Params<T> P, Bufs<T> B) {
+__device__ __forceinline__ void link_pass(const Params<T>& P, const Bufs<T>& B) {
   Ctl* ctl = B.ctl;
-  if (!ctl->rebuild_pending) return;
   const int lp = ctl->lp;
   const int nn = MULTI ? ctl->n_live : P.n;
   const size_t n = (size_t)P.n;
@@ -1971,10 +1994,14 @@ __global__ void link_kernel(Params<T> P, Bufs<T> B) {
   }
 }
 
+template <class T, bool MULTI = false>
+__global__ void link_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending) link_pass<T, MULTI>(P, B);
+}
+
 // 8. clear the key counters for the next rebuild
 template <class T, bool MULTI = false>
-__global__ void clear_keys_kernel(Params<T> P, Bufs<T> B) {
-  if (!B.ctl->rebuild_pending) return;
+__device__ __forceinline__ void clear_keys_pass(const Params<T>& P, const Bufs<T>& B) {
   const int nkeys = MULTI ? B.ctl->key_hi + 1 : P.nkeys;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nkeys; k += gridDim.x * blockDim.x) {
     B.cell_count[k] = 0;
@@ -1982,15 +2009,68 @@ __global__ void clear_keys_kernel(Params<T> P, Bufs<T> B) {
   }
 }
 
+template <class T, bool MULTI = false>
+__global__ void clear_keys_kernel(Params<T> P, Bufs<T> B) {
+  if (B.ctl->rebuild_pending) clear_keys_pass<T, MULTI>(P, B);
+}
+
 // 9. swap to the new buffers
-static __global__ void rebuild_flip_kernel(Ctl* ctl) {
-  if (!ctl->rebuild_pending) return;
+__device__ __forceinline__ void rebuild_flip(Ctl* ctl) {
   ctl->sp ^= 1;
   ctl->lp ^= 1;
   ctl->disp = 0.0f;
   ctl->since = 0;
   ctl->rebuilds += 1;
   ctl->rebuild_pending = 0;
+}
+
+static __global__ void rebuild_flip_kernel(Ctl* ctl) {
+  if (ctl->rebuild_pending) rebuild_flip(ctl);
+}
+
+// The whole pipeline in one block, for small engines: eleven launches less, the
+// same passes in the same order with a block barrier in the place of each.
+template <class T>
+__global__ void __launch_bounds__(kScanThreads) rebuild_small_kernel(Params<T> P, Bufs<T> B) {
+  Ctl* ctl = B.ctl;
+  if (!ctl->rebuild_pending) return;
+  bin_pass<T>(P, B);
+  __syncthreads();
+  int carry = 0;
+  for (int c0 = 0; c0 < P.nkeys; c0 += kScanChunk) {
+    const int base = c0 + (int)threadIdx.x * kScanItems;
+    int v[kScanItems];
+    int local = 0;
+    for (int k = 0; k < kScanItems; ++k) {
+      v[k] = (base + k < P.nkeys) ? B.cell_count[base + k] : 0;
+      local += v[k];
+    }
+    int total;
+    int run = carry + block_exclusive_scan(local, &total);
+    for (int k = 0; k < kScanItems; ++k) {
+      if (base + k < P.nkeys) B.cell_start[base + k] = run;
+      run += v[k];
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) ctl->candidates = 0ull;  // counted anew by the list build
+  __syncthreads();
+  scatter_pass<T>(P, B);
+  __syncthreads();
+  cellsort_pass<T>(P, B);
+  __syncthreads();
+  gather_pass<T>(P, B);
+  __syncthreads();
+  if (P.BMAX > 0) {
+    bond_gather_pass<T>(P, B);
+    __syncthreads();
+  }
+  build_nbr_pass<T>(P, B);
+  __syncthreads();
+  link_pass<T>(P, B);
+  clear_keys_pass<T>(P, B);
+  __syncthreads();
+  if (threadIdx.x == 0) rebuild_flip(ctl);
 }
 
 // ---------------------------------------------------------------------------

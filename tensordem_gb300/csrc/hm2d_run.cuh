@@ -23,6 +23,7 @@
 //                                              one-step  per disc  per pair
 //   300 touching discs x 100 steps, upload        1,924       950       713 us
 //   3,249 dilute discs x 200 steps, upload        2,405       814       852
+//     (667 and 801 with the lists of small engines built by one block)
 //   50,071 touching discs x 100 steps             1,822       954       835
 //   65,535 touching discs x 50 steps, FP64        7,618     6,486     3,938
 //     (3,636 with each pair's effective radius and mass kept)

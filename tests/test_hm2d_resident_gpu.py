@@ -96,6 +96,26 @@ def test_fp64_pairs_with_and_without_room_for_their_constants(hm, skin):
     assert led["status"] == 0 and led["dissipated"] > 0.0
 
 
+# one block up to 4096 discs (FP64 512, bonded 1024, FP64 bonded 128) rebuilds the lists of a small
+# grid; the same discs in a corner of a grid of 40,000 cells sort alike and take the general pipeline
+@pytest.mark.parametrize("precision,side,nx,ny", [(32, 3, 0, 0), (32, 40, 0, 0), (32, 64, 0, 0), (64, 22, 0, 0),
+                                                  (32, 0, 24, 8), (32, 0, 64, 16), (64, 0, 12, 8)])
+def test_one_block_rebuild_equals_the_general_one(hm, precision, side, nx, ny):
+    from dataclasses import replace
+    if side:
+        cfg, st = dense_gas(side, seed=side, precision=precision, walls=5, sigma_v=8.0)
+        bonds, blocks = None, (1, 200)
+    else:
+        cfg, st, *bonds = small_sheet(nx, ny, precision=precision, steps=400, speed=20.0)
+        blocks = (1, 199)
+    small = replace(cfg, ncx=cfg.ncx + 2, ncy=cfg.ncy + 2)
+    assert -(-small.ncx // 32) * -(-small.ncy // 32) * 1024 <= 16384
+    big = replace(cfg, ncx=200, ncy=200)
+    a = _run(hm, small, st, bonds, True, blocks)
+    led = _same(a, _run(hm, big, st, bonds, True, blocks), bonds is not None)
+    assert led["status"] == 0 and (led["rebuilds"] >= 2 or side < 22)
+
+
 def test_indenter_without_bonds(hm):
     """An engine with an indenter but no bond slots takes the bonded build with none."""
     from dataclasses import replace
