@@ -67,8 +67,15 @@ __device__ __forceinline__ void open_instance(const Bufs<T>& B, TileRun<T>& S, i
   S.run = (st & kInstAlive) != 0;
   S.le = eval - S.Q->eval0;
   S.primed = S.le > 0 ? 1 : 0;
-  // quarantine: see batch_kernel
-  const int bad = (st | (st >> kInstRebuildShift)) & (kStatusNonfinite | kStatusEscaped | kStatusCapacity);
+  // quarantine: see batch_kernel. The evaluation in which an instance goes
+  // non-finite is taken by all its tiles, whichever warp opens it after the
+  // mark: its rows are then of one evaluation, and are booked.
+  int bad = (st | (st >> kInstRebuildShift)) & (kStatusNonfinite | kStatusEscaped | kStatusCapacity);
+  if ((st & kStatusNonfinite) && !((st >> kInstRebuildShift) & kStatusNonfinite)) {
+    __threadfence();  // close_tile writes the evaluation before the mark
+    const double at = *reinterpret_cast<volatile double*>(B.iled + (size_t)k * kInstLedger + kInstBadAt);
+    if (at == (double)(S.le + 1)) bad &= ~(int)kStatusNonfinite;
+  }
   S.frozen = S.le >= S.Q->stop || bad != 0;
 }
 
@@ -101,7 +108,11 @@ __device__ __forceinline__ void close_tile(const Bufs<T>& B, TileRun<T>& S, int 
     row[3] = (double)wiy;
     row[4] = (double)wb;
     row[5] = 1.0;
-    if (bad) atomicOr(&B.istate[S.inst], (int)kStatusNonfinite);
+    if (bad) {
+      *reinterpret_cast<volatile double*>(B.iled + (size_t)S.inst * kInstLedger + kInstBadAt) = (double)(S.le + 1);
+      __threadfence();
+      atomicOr(&B.istate[S.inst], (int)kStatusNonfinite);
+    }
   }
 }
 
