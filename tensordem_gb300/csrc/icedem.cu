@@ -531,6 +531,7 @@ __global__ void __launch_bounds__((kClusterWarps + 1) * 32, 1)
 
   int steps_done = 0, buf = 0;
   bool bad = false;
+  double time0 = time;  // start of the step before, which the ledger warps book
   const int total = mode == 1 ? 1 : n_steps;
   cluster.sync();  // every CTA's shared memory is set up
   for (int step = 0; step < total; ++step) {
@@ -584,7 +585,7 @@ __global__ void __launch_bounds__((kClusterWarps + 1) * 32, 1)
     cluster.sync();
     // ---- break test, forces, and the Euler step (dem.py:243-382)
     if (keeper) {
-      if (step > 0) book(time - P.dt, true);
+      if (step > 0) book(time0, true);
     } else {
       for (int q0 = warp * 4; q0 < nd; q0 += warps * 4) {
         const int q = q0 + g;
@@ -817,6 +818,7 @@ __global__ void __launch_bounds__((kClusterWarps + 1) * 32, 1)
     }
     cluster.sync();
     if (copies == 2) buf ^= 1;
+    time0 = time;
     time = time + P.dt;
     steps_done = step + 1;
     const int* fl = sflag + (step & 1) * kMaxCluster;
@@ -857,7 +859,7 @@ __global__ void __launch_bounds__((kClusterWarps + 1) * 32, 1)
   }
   cluster.sync();
   if (!books) return;
-  book(time - P.dt, mode == 0);
+  book(time0, mode == 0);
   double a = -1e300, b = -1e300;
   for (int r = 0; r < nc; ++r) {
     a = fmax(a, peak[2 * r]);
