@@ -561,6 +561,17 @@ struct Engine final : EngineBase {
     return nullptr;
   }
 
+  // The resident kernel of a single step: it has to load what a block of steps
+  // keeps on the chip, so it pays only where the one-step kernel is the slower
+  // form itself. Measured (GB300, us per step(1), one-step / resident): FP64,
+  // 16,384 and 65,535 discs 87 / 46 and 154 / 88; FP32 beyond a disc per thread,
+  // default variant, 1,048,576 and 4,194,304 discs 43 / 39 and 137 / 101; FP32
+  // below, 3,249 to 150,000 discs 24 to 30 / 25 to 32; variants 10 and 11, the same
+  // pipeline in both forms, 1,048,576 discs 28 / 35 and bonded 142 / 147.
+  const RunPlan* resident_once() const {
+    return variant == 0 && run0.fn && (sizeof(T) == 8 || run0.pb == 0) ? &run0 : nullptr;
+  }
+
   bool feat() const { return P.BMAX > 0 || P.irad > T(0); }
   // launch shape of a variant's step kernel (the FP64-sum form has one shape)
   int block_of(int v) const { return sum64 ? 256 : variant_block<T>(v); }
@@ -615,11 +626,11 @@ struct Engine final : EngineBase {
     return TDEM_OK;
   }
 
-  // Adds `step kernel (resident: steps) -> IF(h) { rebuild pipeline }` to graph g.
-  int add_step_and_rebuild(cudaGraph_t g, const cudaGraphNode_t* dep, size_t ndep,
+  // Adds `step kernel (resident r: steps) -> IF(h) { rebuild pipeline }` to graph g.
+  int add_step_and_rebuild(cudaGraph_t g, const RunPlan* r, const cudaGraphNode_t* dep, size_t ndep,
                            cudaGraphConditionalHandle h, cudaGraphConditionalHandle hl, int cond_bits) {
     cudaGraphNode_t knode;
-    if (const RunPlan* r = resident()) {
+    if (r) {
       int discs = r->pb, pairs = r->pairs;
       void* args[] = {&P, &B, &h, &hl, &cond_bits, &discs, &pairs};
       cudaKernelNodeParams kp = {};
@@ -679,27 +690,37 @@ struct Engine final : EngineBase {
     return TDEM_OK;
   }
 
-  // Two graphs: one step (kernel -> IF rebuild), unless the kernel is resident,
-  // and n steps (set target -> WHILE { kernel -> IF rebuild }).
-  int build_graph() {
-    int rc;
-    if (!resident()) {
-      TDEM_CUDA_TRY(&err, cudaGraphCreate(&graph1, 0));
-      TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_reb1, graph1, 0, cudaGraphCondAssignDefault));
-      if ((rc = add_step_and_rebuild(graph1, nullptr, 0, h_reb1, 0, 1))) return rc;
-      TDEM_CUDA_TRY(&err, cudaGraphInstantiate(&exec1, graph1, 0));
-    }
-
-    TDEM_CUDA_TRY(&err, cudaGraphCreate(&graph, 0));
-    TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_loop, graph, 1, cudaGraphCondAssignDefault));
-    long long n0 = 1;
-    void* targs[] = {&B.ctl, &n0};
+  // Adds the node that sets the target n evaluations ahead.
+  int add_target(cudaGraph_t g, long long n, cudaGraphNode_t* node) {
+    void* targs[] = {&B.ctl, &n};
     cudaKernelNodeParams tp = {};
     tp.func = reinterpret_cast<void*>(&set_target_kernel);
     tp.gridDim = dim3(1);
     tp.blockDim = dim3(1);
     tp.kernelParams = targs;
-    TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(&target_node, graph, nullptr, 0, &tp));
+    TDEM_CUDA_TRY(&err, cudaGraphAddKernelNode(node, g, nullptr, 0, &tp));
+    return TDEM_OK;
+  }
+
+  // The graph of one step ([set target ->] kernel -> IF rebuild).
+  int build_once() {
+    int rc;
+    const RunPlan* r = resident_once();
+    cudaGraphNode_t first = nullptr;
+    TDEM_CUDA_TRY(&err, cudaGraphCreate(&graph1, 0));
+    TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_reb1, graph1, 0, cudaGraphCondAssignDefault));
+    if (r && (rc = add_target(graph1, 1, &first))) return rc;
+    if ((rc = add_step_and_rebuild(graph1, r, r ? &first : nullptr, r ? 1 : 0, h_reb1, 0, 1))) return rc;
+    TDEM_CUDA_TRY(&err, cudaGraphInstantiate(&exec1, graph1, 0));
+    return TDEM_OK;
+  }
+
+  // The graph of n steps (set target -> WHILE { kernel -> IF rebuild }).
+  int build_loop() {
+    int rc;
+    TDEM_CUDA_TRY(&err, cudaGraphCreate(&graph, 0));
+    TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_loop, graph, 1, cudaGraphCondAssignDefault));
+    if ((rc = add_target(graph, 1, &target_node))) return rc;
     cudaGraphNodeParams wp = {};
     wp.type = cudaGraphNodeTypeConditional;
     wp.conditional.handle = h_loop;
@@ -709,23 +730,29 @@ struct Engine final : EngineBase {
     TDEM_CUDA_TRY(&err, cudaGraphAddNode(&wnode, graph, &target_node, nullptr, 1, &wp));
     cudaGraph_t body = wp.conditional.phGraph_out[0];
     TDEM_CUDA_TRY(&err, cudaGraphConditionalHandleCreate(&h_reb, body, 0, cudaGraphCondAssignDefault));
-    if ((rc = add_step_and_rebuild(body, nullptr, 0, h_reb, h_loop, 3))) return rc;
+    if ((rc = add_step_and_rebuild(body, resident(), nullptr, 0, h_reb, h_loop, 3))) return rc;
     TDEM_CUDA_TRY(&err, cudaGraphInstantiate(&exec, graph, 0));
     exec_target = 1;
     return TDEM_OK;
   }
 
-  // The step graph, built when it is missing. Where a cooperative node cannot
-  // be instantiated the loop takes the one-step kernel; where no conditional
-  // graph can, steps are plain launches (same results).
-  void ensure_graph() {
-    if (!graph_on || graph_failed || exec) return;
-    if (build_graph() == TDEM_OK) return;
+  // The step graphs (of one step, of n), built when they are missing. Where a
+  // cooperative node cannot be instantiated they take the one-step kernel; where
+  // no conditional graph can, steps are plain launches (same results).
+  void ensure_graph(bool once, bool loop) {
+    if (!graph_on || graph_failed) return;
+    auto build = [&] {
+      int rc = TDEM_OK;
+      if (loop && !exec) rc = build_loop();
+      if (!rc && once && !exec1) rc = build_once();
+      return rc;
+    };
+    if (build() == TDEM_OK) return;
     destroy_graphs();
     if (resident()) {
       run0.fn = runp.fn = nullptr;
       cudaGetLastError();
-      if (build_graph() == TDEM_OK) return;
+      if (build() == TDEM_OK) return;
       destroy_graphs();
     }
     graph_error = err;
@@ -769,25 +796,27 @@ struct Engine final : EngineBase {
   int step(long long n, cudaStream_t s) override {
     if (!has_state) return tdem::fail(&err, TDEM_ERR_STATE, "step before set_state");
     if (n <= 0) {
-      // no step: build the step graph for the current variant now, so that
-      // the next call does not (instantiating it takes ~0.5 s)
-      ensure_graph();
+      // no step: build the step graphs for the current variant now, so that
+      // the next call does not (the process's first takes ~0.5 s)
+      ensure_graph(true, true);
       return TDEM_OK;
     }
     mirror_ok = false;  // rebuild decisions inside the step graph are the device's
-    ensure_graph();
-    const bool in_graph = graph_on && exec;
-    if (!primed && !(in_graph && resident())) {  // the resident kernel primes by itself
+    if (n > 1) ensure_graph(false, true);
+    // a state's first step is plain launches, unless it begins a block of steps
+    // on the resident kernel, which primes by itself
+    if (!primed && !(n > 1 && graph_on && exec && resident())) {
       int rc = prime(s);
       if (rc) return rc;
       --n;
       if (n == 0) return TDEM_OK;
     }
-    if (in_graph) {
-      if (n == 1 && exec1) {
-        TDEM_CUDA_TRY(&err, cudaGraphLaunch(exec1, s));
-        return TDEM_OK;
-      }
+    if (n == 1) ensure_graph(true, false);
+    if (graph_on && n == 1 && exec1) {
+      TDEM_CUDA_TRY(&err, cudaGraphLaunch(exec1, s));
+      return TDEM_OK;
+    }
+    if (graph_on && exec) {
       int rc = set_graph_target(n);
       if (rc) return rc;
       TDEM_CUDA_TRY(&err, cudaGraphLaunch(exec, s));
@@ -888,7 +917,7 @@ struct Engine final : EngineBase {
     v[TDEM_HM_L_REBUILDS] = (double)host_ctl->rebuilds;
     v[TDEM_HM_L_MAX_NEIGHBORS] = (double)host_ctl->max_cnt;
     v[TDEM_HM_L_STATUS] = (double)host_ctl->status;
-    v[TDEM_HM_L_GRAPH] = (exec != nullptr) ? 1.0 : 0.0;
+    v[TDEM_HM_L_GRAPH] = (exec || exec1) ? 1.0 : 0.0;
     v[TDEM_HM_L_VARIANT] = (double)variant;
     std::memcpy(out, v, std::min(count, (int)TDEM_HM_L_COUNT) * sizeof(double));
     return TDEM_OK;
