@@ -530,6 +530,14 @@ int tdem_batch_set_variant(tdem_batch* h, int variant);
 int tdem_batch_get_variant(const tdem_batch* h);
 int tdem_batch_autotune(tdem_batch* h, int steps, float* ms_out, void* stream);
 int tdem_batch_use_graph(tdem_batch* h, int on);
+/* SM clock cycles a grid barrier of the resident step kernel may wait before
+ * the kernel records a timeout and returns (default ~2e9, about a second). For
+ * tests of the failure path (0: every wait runs out that is not over at once).
+ * After it the calls that read states, ledgers or bonds fail with
+ * TDEM_ERR_CUDA, and once one has, so do step, admit and autotune:
+ * the live instances are lost. The batch recovers when the last of them is
+ * retired. */
+int tdem_batch_set_wait_budget(tdem_batch* h, int64_t cycles);
 int tdem_batch_last_error(const tdem_batch* h, char* buf, size_t len);
 
 /* ========================================================================

@@ -228,6 +228,7 @@ def _declare(lib: C.CDLL) -> None:
         "tdem_batch_get_variant": (i32, [vp]),
         "tdem_batch_autotune": (i32, [vp, i32, C.POINTER(C.c_float), vp]),
         "tdem_batch_use_graph": (i32, [vp, i32]),
+        "tdem_batch_set_wait_budget": (i32, [vp, C.c_int64]),
         "tdem_batch_last_error": (i32, [vp, C.c_char_p, C.c_size_t]),
     }
     for name, (res, args) in sig.items():

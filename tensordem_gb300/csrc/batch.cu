@@ -492,6 +492,15 @@ static __global__ void batch_state_kernel(int* istate, int slot, int set, int cl
   istate[slot] = (istate[slot] & ~clear) | set;
 }
 
+// After the last live instance retired: a barrier that ran out of time has
+// nothing left to spoil. The evaluations that it cut off count as the host
+// counted them.
+static __global__ void batch_recover_kernel(Ctl* ctl, long long evals) {
+  if (!(ctl->status & kStatusTimeout)) return;
+  ctl->status &= ~(int)kStatusTimeout;
+  ctl->evals = evals;
+}
+
 static __global__ void batch_key_hi_kernel(Ctl* ctl, int key_hi) { ctl->key_hi = key_hi; }
 
 static __global__ void batch_state_list_kernel(int* istate, const int* ids, int count, int set, int clear) {
@@ -625,6 +634,7 @@ struct BatchBase {
   virtual int get_variant() const = 0;
   virtual int autotune(int steps, cudaStream_t s, float* ms_out) = 0;
   virtual int use_graph(int on) = 0;
+  virtual int set_wait_budget(long long cycles) = 0;
   std::string err;
 };
 
@@ -641,6 +651,8 @@ struct Batch final : BatchBase {
   size_t run_smem = 0;
   bool run_ok = false;  // the resident kernel (variant 0's step loop) can be launched
   bool graph_on = true, graph_failed = false;
+  long long wait_budget = kWaitBudget;  // of the resident kernel's grid barriers, SM clocks
+  bool lost = false;  // such a barrier ran out: the live instances' states are not usable
   // host view of the instances
   struct Inst {
     int state = 0;  // 0 free, 1 live, 2 retired (waiting for the compaction rebuild)
@@ -892,7 +904,7 @@ struct Batch final : BatchBase {
     cudaGraphNode_t knode;
     if (resident()) {
       int n = G.n, bm = G.BMAX, sl = slots;
-      void* args[] = {&B, &h, &hl, &cond_bits, &every, &n, &bm, &sl};
+      void* args[] = {&B, &h, &hl, &cond_bits, &every, &n, &bm, &sl, &wait_budget};
       cudaKernelNodeParams kp = {};
       kp.func = reinterpret_cast<void*>(batch_run_fn<T>());
       kp.gridDim = dim3((unsigned)sms);
@@ -1048,6 +1060,7 @@ struct Batch final : BatchBase {
   int admit(const tdem_hm_config& c, const double* pos, const double* vel, const double* omega, const double* radius,
             const double* mass, const double* inertia, const int* bonds, const double* strength, long long nb,
             int* id, cudaStream_t s) override {
+    if (lost) return fail_lost();
     if (!pos || !vel || !omega || !radius || !mass || !inertia || !id)
       return tdem::fail(&err, TDEM_ERR_BADARG, "admit: null state pointer");
     if (c.n < 1) return tdem::fail(&err, TDEM_ERR_BADARG, "admit: n must be >= 1");
@@ -1178,6 +1191,7 @@ struct Batch final : BatchBase {
   }
 
   int step(long long n, cudaStream_t s) override {
+    if (lost) return fail_lost();
     int rc = settle(s);  // n == 0 settles admissions and retirements and builds the step graph
     if (rc || n < 0) return rc;
     if (graph_on && !graph_failed && !exec && build_graph() != TDEM_OK) {
@@ -1208,10 +1222,16 @@ struct Batch final : BatchBase {
     return TDEM_OK;
   }
 
+  int fail_lost() {
+    return tdem::fail(&err, TDEM_ERR_CUDA,
+                      "a bounded wait (grid barrier) of the batched step ran out: the live instances are lost; "
+                      "retire them all to go on");
+  }
+
   // After a read of the control block: a grid barrier of the steps ran out of time.
   int timed_out() {
-    return (host_ctl->status & kStatusTimeout) ? tdem::fail(&err, TDEM_ERR_CUDA, "a bounded grid barrier timed out")
-                                               : TDEM_OK;
+    if (host_ctl->status & kStatusTimeout) lost = true;
+    return lost ? fail_lost() : TDEM_OK;
   }
 
   int check_id(int id) {
@@ -1364,6 +1384,11 @@ struct Batch final : BatchBase {
     pending_slots.push_back(id);
     pending_keys.emplace_back(I.key_off, I.nkeys);
     need_rebuild = true;
+    if (live == 0) {
+      batch_recover_kernel<<<1, 1, 0, s>>>(B.ctl, evals);
+      TDEM_CUDA_TRY(&err, cudaGetLastError());
+      lost = false;
+    }
     return TDEM_OK;
   }
 
@@ -1387,8 +1412,10 @@ struct Batch final : BatchBase {
     batch_bonds_out_kernel<T><<<grid_items(I.n), kThreads, 0, s>>>(I.par, B, id, dp, ds, want, count_dev);
     TDEM_CUDA_TRY(&err, cudaGetLastError());
     TDEM_CUDA_TRY(&err, cudaMemcpyAsync(count_host, count_dev, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    TDEM_CUDA_TRY(&err, cudaMemcpyAsync(host_ctl, B.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     TDEM_CUDA_TRY(&err, cudaStreamSynchronize(s));
-    const long long got = (long long)*count_host;
+    rc = timed_out();
+    const long long got = rc ? 0 : (long long)*count_host;
     const long long copy = std::min(got, want);
     if (copy > 0) {
       TDEM_CUDA_TRY(&err, cudaMemcpy(pairs, dp, 2 * copy * sizeof(int), cudaMemcpyDeviceToHost));
@@ -1398,6 +1425,7 @@ struct Batch final : BatchBase {
     if (ds) cudaFreeAsync(ds, s);
     TDEM_CUDA_TRY(&err, cudaStreamSynchronize(s));
     if (count) *count = got;
+    if (rc) return rc;
     return got > want ? tdem::fail(&err, TDEM_ERR_CAPACITY, "bond output capacity too small") : TDEM_OK;
   }
 
@@ -1437,6 +1465,7 @@ struct Batch final : BatchBase {
   // and keep the fastest. Plain launches, rebuilds included.
   int autotune(int steps, cudaStream_t s, float* ms_out) override {
     if (steps < 1) return tdem::fail(&err, TDEM_ERR_BADARG, "autotune needs steps >= 1");
+    if (lost) return fail_lost();
     int rc = settle(s);
     if (rc) return rc;
     cudaEvent_t e0, e1;
@@ -1467,6 +1496,13 @@ struct Batch final : BatchBase {
 
   int use_graph(int on) override {
     graph_on = on != 0;
+    return TDEM_OK;
+  }
+
+  int set_wait_budget(long long cycles) override {
+    if (cycles < 0) return tdem::fail(&err, TDEM_ERR_BADARG, "wait budget must be >= 0");
+    wait_budget = cycles;
+    destroy_graphs();  // the step graph holds it by value
     return TDEM_OK;
   }
 };
@@ -1611,6 +1647,11 @@ int tdem_batch_autotune(tdem_batch* h, int steps, float* ms_out, void* stream) {
 int tdem_batch_use_graph(tdem_batch* h, int on) {
   if (!h) return TDEM_ERR_BADARG;
   return h->e->use_graph(on);
+}
+
+int tdem_batch_set_wait_budget(tdem_batch* h, int64_t cycles) {
+  if (!h) return TDEM_ERR_BADARG;
+  return h->e->set_wait_budget((long long)cycles);
 }
 
 int tdem_batch_last_error(const tdem_batch* h, char* buf, size_t len) {

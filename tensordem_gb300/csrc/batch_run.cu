@@ -372,7 +372,7 @@ __device__ __forceinline__ void book_instance(const Bufs<T>& B, int k, long long
 template <class T>
 __global__ void __launch_bounds__(kBatchRunBlock<T>, 1)
     batch_run_kernel(Bufs<T> B, cudaGraphConditionalHandle h_rebuild, cudaGraphConditionalHandle h_loop, int use_cond,
-                     int rebuild_every, int n, int BM, int slots) {
+                     int rebuild_every, int n, int BM, int slots, long long budget) {
   constexpr int NW = kBatchRunBlock<T> / 32;
   extern __shared__ __align__(16) unsigned char run_smem[];
   __shared__ alignas(16) Params<T> s_par[2 * NW];
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kBatchRunBlock<T>, 1)
   while (true) {
     if (strains) {
       strain_tiles<T>(B, run_smem, n, BM, fb, fe, sp, lp);
-      grid_barrier(ctl, gridDim.x, epoch++, nullptr, nullptr, kWaitBudget, s_out);
+      grid_barrier(ctl, gridDim.x, epoch++, nullptr, nullptr, budget, s_out);
       if (s_out[3]) {
         late = true;
         break;
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kBatchRunBlock<T>, 1)
     if (eval > first) book(eval - 1);
     const int k1 = k3 == 2 ? 0 : k3 + 1;
     if (t == 0) s_vmax[k1] = 0u;  // the next evaluation's slot: last read an evaluation ago
-    grid_barrier(ctl, gridDim.x, epoch++, &s_vmax[k3], nullptr, kWaitBudget, s_out);
+    grid_barrier(ctl, gridDim.x, epoch++, &s_vmax[k3], nullptr, budget, s_out);
     if (s_out[3]) {
       late = true;
       break;

@@ -25,7 +25,8 @@ inline size_t batch_run_smem(int bmax, bool prem, bool fp32) {
 }
 
 template <class T>
-using BatchRunFn = void (*)(Bufs<T>, cudaGraphConditionalHandle, cudaGraphConditionalHandle, int, int, int, int, int);
+using BatchRunFn = void (*)(Bufs<T>, cudaGraphConditionalHandle, cudaGraphConditionalHandle, int, int, int, int, int,
+                            long long);
 template <class T>
 BatchRunFn<T> batch_run_fn();
 
