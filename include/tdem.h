@@ -351,13 +351,14 @@ int tdem_hm_rebuild_pending(tdem_hm* h, void* stream);
 int tdem_hm_num_variants(void);
 int tdem_hm_set_variant(tdem_hm* h, int variant);
 int tdem_hm_get_variant(const tdem_hm* h);
-/* SM clock cycles a bounded wait of the bulk-copy step kernels (variants 4-6)
- * may take before the kernel records a timeout, drains its copies in flight
- * and returns (default ~2e9, about a second). For tests of the failure path:
- * a budget of 0 makes each wait a single non-blocking probe of the copy it
- * waits for, so the waits run out; the next status check then fails
- * with TDEM_ERR_CUDA, and the engine recovers with set_state. No counterpart
- * in the reference (it has no device waits). */
+/* SM clock cycles a bounded wait may take, of the bulk-copy step kernels
+ * (variants 4-6) and of the resident step kernels' grid barrier (the default
+ * loop, and that of variants 10 and 11), before the kernel records a timeout,
+ * drains its copies in flight and returns (default ~2e9, about a second). For
+ * tests of the failure path: a budget of 0 makes each wait a single
+ * non-blocking probe of what it waits for, so the waits run out; the next
+ * status check then fails with TDEM_ERR_CUDA, and the engine recovers with
+ * set_state. No counterpart in the reference (it has no device waits). */
 int tdem_hm_set_wait_budget(tdem_hm* h, int64_t cycles);
 int tdem_hm_autotune(tdem_hm* h, int steps, float* ms_out, void* stream);
 

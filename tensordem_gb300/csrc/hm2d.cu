@@ -933,7 +933,9 @@ struct Engine final : EngineBase {
       return tdem::fail(&err, TDEM_ERR_CAPACITY,
                         "neighbour capacity exceeded (max_neighbors=" + std::to_string(P.W) + ")");
     if (st & kStatusEscaped) return tdem::fail(&err, TDEM_ERR_CAPACITY, "a particle left the cell grid");
-    if (st & kStatusTimeout) return tdem::fail(&err, TDEM_ERR_CUDA, "a bounded wait on a bulk copy timed out");
+    if (st & kStatusTimeout)
+      return tdem::fail(&err, TDEM_ERR_CUDA, std::string("a bounded wait on a ") +
+                                                 (resident() ? "grid barrier" : "bulk copy") + " timed out");
     if (st & kStatusInertia)
       return tdem::fail(&err, TDEM_ERR_BADARG, "moment of inertia must be inertia_factor * m * r^2");
     return TDEM_OK;

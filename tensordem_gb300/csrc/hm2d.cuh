@@ -50,7 +50,7 @@ enum Status : int {
   kStatusNonfinite = 2,  // non-finite position or velocity
   kStatusEscaped = 4,    // a particle left the cell grid by more than a cell
   kStatusInertia = 8,    // an uploaded moment of inertia was not kappa m r^2
-  kStatusTimeout = 16,   // a bounded wait on a bulk copy ran out
+  kStatusTimeout = 16,   // a bounded wait (bulk copy, grid barrier) ran out
 };
 
 template <class T>
@@ -101,8 +101,8 @@ struct Params {
   float eps_t_lo, eps_t_hi, eps_s_lo, eps_s_hi;
   // indenter centre at evaluation 0 and its displacement per evaluation
   float ind_x0f, ind_y0f, ind_dxf, ind_dyf;
-  // SM clock cycles a bounded wait of the bulk-copy kernels may take (about
-  // a second by default; tests of the failure path shorten it)
+  // SM clock cycles a bounded wait of the bulk-copy and the resident kernels may
+  // take (about a second by default; tests of the failure path shorten it)
   long long wait_budget;
 };
 
