@@ -1228,9 +1228,10 @@ __global__ void __launch_bounds__(kBlock, kBlocks) icedem3d_kernel(tdem_icedem3d
           // spherical indenter (dem3d.py:1519-1532)
           {
             const double dx = px - tpx, dy = py - tpy, dz = pz - tpz;
-            // out of reach it adds zero: screened in FP32 (a few ulp against a 1e-3 guard band)
+            // out of reach it adds zero: screened in FP32 (a few ulp against a 1e-3 guard band,
+            // and an absolute one where the squares underflow)
             const float sx = (float)dx, sy = (float)dy, sz = (float)dz, sr = (float)(P.radius + P.tool_radius);
-            if (!(sx * sx + sy * sy + sz * sz > sr * sr * 1.001f)) {
+            if (!(sx * sx + sy * sy + sz * sz > sr * sr * 1.001f + 1e-30f)) {
               const double dist = norm3(dx, dy, dz);
               double nx = 0.0, ny = 0.0, nz = -1.0;
               if (dist > kEps) {
