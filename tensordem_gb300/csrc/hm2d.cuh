@@ -150,7 +150,7 @@ struct Ctl {
   // counts them across launches), zeroed one barrier ahead
   unsigned epoch;
   unsigned entries[2];     // indenter partials of the even and odd evaluations
-  unsigned long long candidates;  // candidate slots of all lists (the last rebuild's)
+  unsigned candidates;     // candidate slots of all lists (the last rebuild's, mod 2^32: read for engines far below)
   alignas(128) GridWord word[3];
 };
 
