@@ -38,24 +38,44 @@ __device__ __forceinline__ T lanes_sum(T x) {
   return x;
 }
 
-// What a warp keeps across its tiles of one evaluation.
+// What a warp keeps across its tiles of one evaluation. No more than this: the
+// bonded build is short of registers (an instance's evaluation index, its state
+// in two words and the evaluation that these were read in, kept as well, were 7%
+// of a step of 256 runs with 1.16M discs).
 template <class T>
 struct TileRun {
-  Params<T>* Q;   // the open instance's parameters (shared memory, per warp)
-  int inst;       // the open instance, -1: none
-  long long at;   // the evaluation its state word was read in
-  bool run, frozen;
-  int primed;
-  long long le;   // the instance's own evaluation index
-  float vmax;     // max over the thread's discs of (|v| dt / rebuild displacement)^2
+  Params<T>* Q;  // the open instance's parameters (shared memory, per warp)
+  int inst;      // the open instance, -1: none
+  int go;        // -1: to be read in this evaluation, 0: retired, 1: frozen, 2: stepped
+  float vmax;    // max over the thread's discs of (|v| dt / rebuild displacement)^2
 };
+
+// Marks instance k non-finite in the batch's evaluation eval: the evaluation
+// first, then the bit that says to look for it. (No memory clobber, here and
+// below: nothing else needs these orders.)
+template <class T>
+__device__ __forceinline__ void mark_bad(const Bufs<T>& B, int k, long long eval) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;\n\tred.release.gpu.global.or.b32 [%2], %3;" ::"l"(
+                   B.iled + (size_t)k * kInstLedger + kInstBadAt),
+               "d"((double)(eval + 1)), "l"(B.istate + k), "r"((int)kStatusNonfinite));
+}
+
+// What mark_bad wrote, after its bit was seen: the evaluation after, 0 if the
+// bit is not a resident step's.
+template <class T>
+__device__ __forceinline__ double marked_at(const Bufs<T>& B, int k) {
+  double at;
+  asm volatile("{\n\t.reg .b32 t;\n\tld.acquire.gpu.global.b32 t, [%1];\n\tld.relaxed.gpu.global.f64 %0, [%2];\n\t}"
+               : "=d"(at)
+               : "l"(B.istate + k), "l"(B.iled + (size_t)k * kInstLedger + kInstBadAt));
+  return at;
+}
 
 template <class T>
 __device__ __forceinline__ void open_instance(const Bufs<T>& B, TileRun<T>& S, int k, long long eval) {
-  if (k == S.inst && S.at == eval) return;
+  if (k == S.inst && S.go >= 0) return;
   const int lane = threadIdx.x & 31;
   const int st = *reinterpret_cast<volatile int*>(&B.istate[k]);
-  S.at = eval;
   if (k != S.inst) {
     S.inst = k;
     __syncwarp();
@@ -64,27 +84,22 @@ __device__ __forceinline__ void open_instance(const Bufs<T>& B, TileRun<T>& S, i
     for (int w = lane; w < (int)(sizeof(Params<T>) / 4); w += 32) dst[w] = src[w];
     __syncwarp();
   }
-  S.run = (st & kInstAlive) != 0;
-  S.le = eval - S.Q->eval0;
-  S.primed = S.le > 0 ? 1 : 0;
   // quarantine: see batch_kernel. The evaluation in which an instance goes
   // non-finite is taken by all its tiles, whichever warp opens it after the
   // mark: its rows are then of one evaluation, and are booked.
   int bad = (st | (st >> kInstRebuildShift)) & (kStatusNonfinite | kStatusEscaped | kStatusCapacity);
-  if ((st & kStatusNonfinite) && !((st >> kInstRebuildShift) & kStatusNonfinite)) {
-    __threadfence();  // close_tile writes the evaluation before the mark
-    const double at = *reinterpret_cast<volatile double*>(B.iled + (size_t)k * kInstLedger + kInstBadAt);
-    if (at == (double)(S.le + 1)) bad &= ~(int)kStatusNonfinite;
-  }
-  S.frozen = S.le >= S.Q->stop || bad != 0;
+  if ((st & kStatusNonfinite) && !((st >> kInstRebuildShift) & kStatusNonfinite) &&
+      marked_at(B, k) == (double)(eval + 1))
+    bad &= ~(int)kStatusNonfinite;
+  S.go = !(st & kInstAlive) ? 0 : eval - S.Q->eval0 >= S.Q->stop || bad != 0 ? 1 : 2;
 }
 
 // One disc of the tile is done: the tile's ledger row and the speed bound.
 template <class T, bool FEAT>
-__device__ __forceinline__ void close_tile(const Bufs<T>& B, TileRun<T>& S, int tile, int par, bool stepped,
+__device__ __forceinline__ void close_tile(const Bufs<T>& B, TileRun<T>& S, int tile, long long eval, bool stepped,
                                            const ThreadLedger<T>& L) {
   const int lane = threadIdx.x & 31;
-  double* row = B.tpart + (size_t)tile * kTileVals + par * kRowHalf;
+  double* row = B.tpart + (size_t)tile * kTileVals + (int)(eval & 1) * kRowHalf;
   if (!stepped) {
     if (lane == 0) row[5] = 0.0;
     return;
@@ -108,11 +123,7 @@ __device__ __forceinline__ void close_tile(const Bufs<T>& B, TileRun<T>& S, int 
     row[3] = (double)wiy;
     row[4] = (double)wb;
     row[5] = 1.0;
-    if (bad) {
-      *reinterpret_cast<volatile double*>(B.iled + (size_t)S.inst * kInstLedger + kInstBadAt) = (double)(S.le + 1);
-      __threadfence();
-      atomicOr(&B.istate[S.inst], (int)kStatusNonfinite);
-    }
+    if (bad) mark_bad(B, S.inst, eval);
   }
 }
 
@@ -128,20 +139,20 @@ __device__ __forceinline__ void force_tiles_plain(const Bufs<T>& B, TileRun<T>& 
     const int i = d.y + lane;
     const bool on = lane < d.z;
     ThreadLedger<T> L;
-    if (on && S.run) {
+    if (on && S.go) {
       const V4<T> p = fetch.p(i), v = fetch.v(i);
-      if (S.frozen) {
+      if (S.go == 1) {
         B.pos[sp ^ 1][i] = p;
         B.vel[sp ^ 1][i] = v;
       } else {
         const uint4 hd = B.head[lp][i];
         V4<T> q0{}, q1{}, q2{};
         load_head_partners<T>(fetch, hd, q0, q1, q2);
-        process_particle_q<T, kBatch, FEAT, PlainFetch<T>>(*S.Q, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, S.primed,
-                                                           S.le, L);
+        process_particle_q<T, kBatch, FEAT, PlainFetch<T>>(*S.Q, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, eval > S.Q->eval0 ? 1 : 0,
+                                                           eval - S.Q->eval0, L);
       }
     }
-    close_tile<T, FEAT>(B, S, tile, (int)(eval & 1), S.run && !S.frozen, L);
+    close_tile<T, FEAT>(B, S, tile, eval, S.go == 2, L);
   }
 }
 
@@ -216,10 +227,10 @@ __device__ __forceinline__ void force_tiles(const Bufs<T>& B, TileRun<T>& S, uns
       cp_wait<2>();  // this tile's partners have landed
       open_instance<T>(B, S, d0.x, eval);
       ThreadLedger<T> L;
-      if (lane < d0.z && S.run) {
+      if (lane < d0.z && S.go) {
         const int i = d0.y + lane;
         const V4<T> p = spos[s * BL + t], v = svel[s * BL + t];
-        if (S.frozen) {
+        if (S.go == 1) {
           B.pos[sp ^ 1][i] = p;
           B.vel[sp ^ 1][i] = v;
         } else {
@@ -233,16 +244,16 @@ __device__ __forceinline__ void force_tiles(const Bufs<T>& B, TileRun<T>& S, uns
           const float2 rm = pr ? srem[s * BL + t] : make_float2(0.0f, 0.0f);
           if constexpr (FEAT) {
             process_particle_q<T, kBatch, true, PlainFetch<T>, false, true>(
-                *S.Q, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, S.primed, S.le, L, &rm, sbw + s * BM * BL + t, BL,
+                *S.Q, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2, eval > S.Q->eval0 ? 1 : 0, eval - S.Q->eval0, L, &rm, sbw + s * BM * BL + t, BL,
                 BM > 0 ? sbc[s * BL + t] : 0, BM > 0 ? ssi[s * BL + t] : T(0));
           } else {
             process_particle_q<T, kBatch, false, PlainFetch<T>>(*S.Q, B, fetch, sp, lp, i, p, v, hd, q0, q1, q2,
-                                                                S.primed, S.le, L, &rm);
+                                                                eval > S.Q->eval0 ? 1 : 0, eval - S.Q->eval0, L, &rm);
           }
         }
       }
       __syncwarp();
-      close_tile<T, FEAT>(B, S, tile, (int)(eval & 1), S.run && !S.frozen, L);
+      close_tile<T, FEAT>(B, S, tile, eval, S.go == 2, L);
       d0 = d1;
       d1 = d2;
       d2 = d3;
@@ -413,7 +424,7 @@ __global__ void __launch_bounds__(kBatchRunBlock<T>, 1)
     }
   };
   // open instances of the bonded and the granular range
-  TileRun<T> S{&s_par[t >> 5], -1, -1, false, false, 0, 0, 0.0f}, G{&s_par[NW + (t >> 5)], -1, -1, false, false, 0, 0, 0.0f};
+  TileRun<T> S{&s_par[t >> 5], -1, -1, 0.0f}, G{&s_par[NW + (t >> 5)], -1, -1, 0.0f};
   int k3 = 0, rebuild = 0;
   bool late = false;
   __syncthreads();
@@ -427,6 +438,7 @@ __global__ void __launch_bounds__(kBatchRunBlock<T>, 1)
       }
     }
     S.vmax = G.vmax = 0.0f;
+    S.go = G.go = -1;  // state words are read anew
     force_tiles<T, true>(B, S, run_smem, n, BM, fb, fe, sp, lp, eval);
     force_tiles<T, false>(B, G, run_smem, n, BM, pb, pe, sp, lp, eval);
     const unsigned bits = __reduce_max_sync(kAll, __float_as_uint(fmaxf(S.vmax, G.vmax)));

@@ -162,7 +162,7 @@ constexpr int kInstRebuildShift = 16;  // Status bits found by a rebuild (bits 1
 constexpr int kTile = 32;
 constexpr int kTileVals = 12;        // per-tile ledger partial row
 constexpr int kInstLedger = 24;      // per-instance ledger row (doubles)
-constexpr int kInstBadAt = 18;       // its entry: evaluations taken when a resident step went non-finite (0: none)
+constexpr int kInstBadAt = 18;       // its entry: the batch evaluation after the one that went non-finite (0: none)
 
 template <class T>
 struct Bufs {
