@@ -104,7 +104,7 @@ class Batch:
         _lib.check(rc, None, "tdem_batch_create")
         self._h = h
         self.sizes: dict[int, int] = {}
-        # TDEM_GRAPH=0: plain launches (visible to profilers), same results
+        # TDEM_GRAPH=0: the one-step kernels as plain launches (visible to profilers), same results
         if os.environ.get("TDEM_GRAPH", "1") == "0":
             self.use_graph(False)
 

@@ -18,10 +18,10 @@
 //
 // Measured (GB300, a block of steps with its ledgers and two states read;
 // one-step launches -> this): 32 runs of 100 to 2,000 discs (22,673 discs) x
-// 100 steps 10,268 -> 2,220 us (99 -> 20 us a step: 91 chunks of 8 tiles had
+// 100 steps 10,625 -> 2,209 us (99 -> 19 us a step: 91 chunks of 8 tiles had
 // kept 91 of 4,864 warps busy); 256 runs of 100 to 20,000 discs (1.16M) x 40
-// steps 12,487 -> 7,080 us (6,950 with the lean contact test; L2 prefetches of
-// the next tile's bond rows cost 9% of it).
+// steps 12,832 -> 6,696 us (310 -> 124 us a step; L2 prefetches of the next tile's
+// bond rows cost 9% of it).
 #include "batch_run.cuh"
 
 namespace tdem {

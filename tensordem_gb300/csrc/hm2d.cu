@@ -492,7 +492,9 @@ struct Engine final : EngineBase {
   // thread of the chip. One block while that costs no more than a grid
   // barrier; else blocks of at least 128 discs (one warp per scheduler), as
   // many as the discs need, one per SM; the big build only when the other
-  // does not hold them.
+  // does not hold them (its spills cost more than its threads give: us a step,
+  // other build / big, 50,071 touching discs 6.8 / 8.0, 22,500 dilute 3.0 / 3.3,
+  // 30,000 bonded 10.5 / 10.9; 16,384 touching discs in FP64 24.9 / 23.5).
   int plan_run(int dev, int sms) {
     int smem_max = 0, coop = 0;
     TDEM_CUDA_TRY(&err, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));

@@ -102,7 +102,14 @@ constexpr int run_block(bool feat, bool big) {
 }
 
 // Discs of a block: at least kRunDiscs in a grid; up to kRunLocal (with bonds
-// kRunLocalBonds) stay in one block.
+// kRunLocalBonds) stay in one block. Measured (GB300, us a step):
+//   blocks of 32 / 64 / 128 / 256 discs: 3,249 touching discs 4.9 / 5.0 / 5.0 / 5.8,
+//     dilute 2.5 / 2.4 / 2.5 / 2.6, 2,328 bonded 10.4 / 10.0 / 10.0 / 10.3, 182
+//     bonded 10.5 / 9.6 / 9.5 / 9.5; in FP64 3,249 touching discs 16.1 / 17.2 / 25.0 /
+//     39.1 (smaller blocks would pay there), 16,384 24.9 / 24.9 / 24.9 / 38.7;
+//   one block / a grid: 256 touching discs 3.9 / 4.6, 400 4.7 / 4.9, 506 4.8 / 4.6;
+//     256 dilute 1.1 / 2.3, 484 1.3 / 2.5; 128 bonded 7.6 / 10.0 (182 would still gain,
+//     7.6 / 9.5); FP64, 256 touching discs 29.9 / 20.4 (a grid would pay from there).
 constexpr int kRunDiscs = 128;
 constexpr int kRunLocal = 512;
 constexpr int kRunLocalBonds = 128;

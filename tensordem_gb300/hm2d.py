@@ -179,8 +179,8 @@ class HM2D:
         self._h = h
         self.steps = 0
         self._anchor = torch.zeros(1, device=self.device)  # the device of the torch ops
-        # TDEM_GRAPH=0 runs steps as plain launches (profilers cannot see
-        # kernels inside conditional CUDA graphs); results are identical.
+        # TDEM_GRAPH=0 runs the one-step kernels as plain launches (profilers cannot
+        # see kernels inside conditional CUDA graphs); results are identical.
         if os.environ.get("TDEM_GRAPH", "1") == "0":
             self.use_graph(False)
 
@@ -225,8 +225,8 @@ class HM2D:
 
     def step(self, n_steps: int = 1, *, check: bool = True) -> None:
         """Advance n velocity-Verlet steps (one graph launch). ``step(0)``
-        only builds the step graph for the current variant (about half a
-        second), which the first stepping call would otherwise pay."""
+        only builds the step graphs for the current variant (about half a
+        second the first time), which the first stepping calls would otherwise pay."""
         from . import ops
         with torch.cuda.device(self.device):
             ops.hm_step(self._h.value, int(n_steps), self._anchor)
