@@ -273,9 +273,10 @@ int tdem_hm_set_state(tdem_hm* h, const double* pos, const double* vel, const do
 /* Advance n velocity-Verlet steps (FloeBed.step, kernel.py:410-419), list
  * rebuilds and history remap included (kernel.py:230-274). Asynchronous:
  * check tdem_hm_status afterwards. n_steps == 0 steps nothing and builds the
- * step graphs (of one step, of many) for the current variant if they are not
- * built yet (the first stepping calls after creation or a variant change
- * otherwise pay that, about half a second the first time in a process). */
+ * step graph for the current variant if it is not built yet (the first
+ * stepping call after creation or a variant change otherwise pays that, about
+ * half a second the first time in a process). Where single steps have a graph
+ * of their own (about 0.1 ms), the first of them builds it. */
 int tdem_hm_step(tdem_hm* h, int64_t n_steps, void* stream);
 
 /* Integer-time state in original order: positions, velocities, omega, total

@@ -798,9 +798,11 @@ struct Engine final : EngineBase {
   int step(long long n, cudaStream_t s) override {
     if (!has_state) return tdem::fail(&err, TDEM_ERR_STATE, "step before set_state");
     if (n <= 0) {
-      // no step: build the step graphs for the current variant now, so that
-      // the next call does not (the process's first takes ~0.5 s)
-      ensure_graph(true, true);
+      // no step: build the step graph for the current variant now, so that the
+      // next call does not (the process's first takes ~0.5 s). A resident loop has a
+      // graph of its own for single steps, which the first of them builds: it costs
+      // some 0.1 ms, an eighth of preparing 300 discs, and most callers step in blocks.
+      ensure_graph(!resident(), true);
       return TDEM_OK;
     }
     mirror_ok = false;  // rebuild decisions inside the step graph are the device's

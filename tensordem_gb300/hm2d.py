@@ -225,8 +225,8 @@ class HM2D:
 
     def step(self, n_steps: int = 1, *, check: bool = True) -> None:
         """Advance n velocity-Verlet steps (one graph launch). ``step(0)``
-        only builds the step graphs for the current variant (about half a
-        second the first time), which the first stepping calls would otherwise pay."""
+        only builds the step graph for the current variant (about half a
+        second the first time), which the first stepping call would otherwise pay."""
         from . import ops
         with torch.cuda.device(self.device):
             ops.hm_step(self._h.value, int(n_steps), self._anchor)
